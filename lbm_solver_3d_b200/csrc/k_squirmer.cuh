@@ -11,6 +11,9 @@
 //                reference's order-dependent semantics, then a rebuild of the
 //                boundary-link list (fluid nodes next to the sphere, in
 //                ascending node order) and of the near-particle flag bits.
+//                A step that changes at most SQ_FEW nodes takes a short way
+//                through the same steps (remap_few); the walk over the whole
+//                box runs when the candidate list is rebuilt or more change.
 //   stage LOOP : time-loop bookkeeping of src/main.cpp:60-64: schedule the
 //                mass correction of correction steps (applied by the next
 //                stream kernel on load), record the trajectory row, and set
@@ -37,9 +40,16 @@ namespace lbmgpu {
 
 constexpr int SQ_THREADS = 512;
 constexpr int SQ_BATCH = 256;
-constexpr int SQ_SORT_CAP = 2048;
-constexpr int SQ_GROUP = 4;         // remap candidates tested per thread with their loads in flight together   // changes ordered in shared memory (3 ints each)
+constexpr int SQ_SORT_CAP = 2048;   // changes ordered in shared memory (3 ints each)
+constexpr int SQ_GROUP = 4;         // remap candidates tested per thread with their loads in flight together
+constexpr int SQ_PRE = 6;           // candidates per thread fetched ahead: 3072 of them, the shell up to R = 8
+constexpr int SQ_FEW = 32;          // changed nodes that remap_few orders: one warp
+constexpr int SQ_FEW_LINKS = 4096;  // boundary links that remap_few edits in shared memory (R up to about 12)
 constexpr int STAGE_BODY = 1, STAGE_REMAP = 2, STAGE_LOOP = 4, STAGE_FORCE = 8;
+// The launch directly follows a zone kernel that had itself waited for the
+// update before: this update may read what that one wrote (its state, the
+// candidate list, the node types) before its own pdl_wait.
+constexpr int STAGE_PRE = 16;
 
 struct SqArgs {
     void* f;
@@ -89,32 +99,48 @@ __device__ __forceinline__ double soft_wall_force(double h, double eps, double F
     return eps * FS * s * s;
 }
 
-// Deterministic block sum of ncols (<= 8) columns over rows of a strided array.
+// Deterministic block sum of NC (<= 8) columns over rows of a strided array:
+// each thread its rows in order, a shuffle tree per warp, the warps in order.
+// Short loops: the code runs once per step, from a cold instruction cache.
 template <int NC>
-__device__ void block_sum_rows(const double* base, int rows, int stride, int col0, double* out_sh) {
+__device__ __forceinline__ void block_sum_rows(const double* base, int rows, int stride, int col0, double* out_sh) {
     __shared__ double red[SQ_THREADS / 32][8];
     double acc[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) acc[c] = 0.0;
-    for (int k = threadIdx.x; k < rows; k += SQ_THREADS) {
+    constexpr int U = NC > 1 ? 1 : 8;   // rows per thread with their loads in flight together
+#pragma unroll 1
+    for (int k0 = threadIdx.x; k0 < rows; k0 += U * SQ_THREADS) {
+        double v[U][NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) acc[c] += base[(size_t)k * stride + col0 + c];
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const int k = k0 + u * SQ_THREADS;
+                v[u][c] = k < rows ? base[(size_t)k * stride + col0 + c] : 0.0;
+            }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k0 + u * SQ_THREADS < rows)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) acc[c] += v[u][c];
     }
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-    for (int c = 0; c < NC; ++c)
-        for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_down_sync(0xffffffffu, acc[c], o);
+        for (int c = 0; c < NC; ++c) acc[c] += __shfl_down_sync(0xffffffffu, acc[c], o);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (lane == 0)
 #pragma unroll
         for (int c = 0; c < NC; ++c) red[wid][c] = acc[c];
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < NC) {   // one thread per column, the warps in order
+        double v[SQ_THREADS / 32], s = 0.0;
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            double s = 0.0;
-            for (int w = 0; w < SQ_THREADS / 32; ++w) s += red[w][c];
-            out_sh[c] = s;
-        }
+        for (int w = 0; w < SQ_THREADS / 32; ++w) v[w] = red[w][threadIdx.x];
+#pragma unroll
+        for (int w = 0; w < SQ_THREADS / 32; ++w) s += v[w];
+        out_sh[threadIdx.x] = s;
     }
     __syncthreads();
 }
@@ -133,545 +159,940 @@ struct AxisRange {
 
 static_assert(3 * SQ_SORT_CAP * sizeof(int) <= SQ_BATCH * sizeof(ChgSh), "the change sort fits the batch stage");
 
+// What one update keeps in shared memory besides the batch stage.
+struct SqShared {
+    SqState s;
+    double sums[8];
+    double mass_delta;            // stored mass that covered and uncovered nodes take or bring (correction steps)
+    long long dfluid;
+    int total, box[6], rebuild, ncand, few, nins, nrem;
+    int wbox[3];                  // the box's corner wrapped into the lattice
+    int ci[3];                    // the centre: the node below it (wrapped) ...
+    float cf[3];                  // ... and the fraction of a cell above that
+    typename cub::BlockScan<int, SQ_THREADS>::TempStorage scan;
+};
+
+// ---------------------------------------------------------------------------
+//  remap_few: the remap of a step that changes at most SQ_FEW nodes and a link
+//  list of at most SQ_FEW_LINKS entries, which is nearly every step (a sphere
+//  moving U cells a step changes about 2 pi R^2 U nodes: 0.3 to 3 in the
+//  channels here). Everything stays in shared memory, one warp replays the
+//  changes, and the list is edited (entries gained and lost near the changed
+//  nodes) instead of being rebuilt by two walks over the sphere's box.
+//  The update is bound by latency: it runs once per step on one SM, so besides
+//  its dependent loads it waits for its own instructions, which come from a
+//  cold cache (straight-line code cost 140 cycles per 128 bytes of it). Hence
+//  short loops with the tasks spread over the threads, and divisions done once
+//  for all components. Whole update, launched back to back: 14.9 -> 8.3 us
+//  (64x34x32, R = 4), 13.6 -> 8.5 us (128x64x64, R = 6), 21.7 -> 11.3 us
+//  (256x128x128, R = 8); a step with changes 55-68 us before, 15-22 us with
+//  this. Channel step 37.8 -> 28.2 us, slit step 38.9 -> 34.2 us.
+// ---------------------------------------------------------------------------
+struct FewSh {
+    double pop[SQ_FEW][Q];        // covered: the node's stored numbers; uncovered: the refilled ones
+    double nbrho[SQ_FEW][Q];
+    double part[SQ_FEW][6];       // what the change adds to Fc, Tc
+    double r[SQ_FEW][3], ub[SQ_FEW][3], rr[SQ_FEW], mass[SQ_FEW];
+    unsigned fnode[SQ_FEW];       // changed nodes as found
+    int fx[SQ_FEW], fy[SQ_FEW], fz[SQ_FEW], fkind[SQ_FEW], fkey[SQ_FEW];
+    unsigned node[SQ_FEW];        // in the order of their first visit in the box
+    int x[SQ_FEW], y[SQ_FEW], z[SQ_FEW], kind[SQ_FEW];   // kind: 1 covered, 2 uncovered
+    int nbord[SQ_FEW][Q];         // the change that neighbour j is, or -1
+    uint8_t flag[SQ_FEW][Q];      // flag byte of neighbour j (0: the node) before the changes
+    uint8_t near[SQ_FEW][Q];      // neighbour j (0: the node) has a PARTICLE neighbour after them
+    unsigned ins[SQ_FEW * Q], rem[SQ_FEW * Q];           // nodes that enter / leave the link list
+    int list[SQ_FEW_LINKS];
+};
+// The candidates fetched ahead, each written and read by the same thread (in
+// registers they took the update to 128 a thread and spills).
+struct CandSh {
+    unsigned n[SQ_PRE * SQ_THREADS];
+    int x[SQ_PRE * SQ_THREADS];
+    unsigned yz[SQ_PRE * SQ_THREADS];   // y, z < 65536
+    uint8_t ty[SQ_PRE * SQ_THREADS];
+};
+constexpr size_t FEW_BYTES = (sizeof(FewSh) + 15) / 16 * 16;
+static_assert(FEW_BYTES + sizeof(CandSh) <= SQ_BATCH * sizeof(ChgSh),
+              "the few-changes stage and the candidates fit the batch stage");
+
+// index distance a - b on an axis of n nodes, as -1, 0, 1 for neighbours (with
+// wrap) and something else otherwise
+__device__ __forceinline__ int axis_delta(int a, int b, int n) {
+    const int d = a - b;
+    return d == n - 1 ? -1 : (d == 1 - n ? 1 : d);
+}
+__device__ __forceinline__ bool near_or_same(const Lattice& L, const FewSh& w, int e, int x, int y, int z) {
+    const int dx = abs(axis_delta(x, w.x[e], L.nx)), dy = abs(axis_delta(y, w.y[e], L.ny)),
+              dz = abs(axis_delta(z, w.z[e], L.nz));
+    return dx <= 1 && dy <= 1 && dz <= 1 && dx + dy + dz < 3;
+}
+__device__ __forceinline__ int wrap1(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
+
+// Called by all threads; w.f* hold the nfew changes in any order.
 template <class S>
-__device__ void squirmer_update(const Lattice& L, const SqArgs& a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ChgSh* ch = reinterpret_cast<ChgSh*>(smem_raw);
-    __shared__ SqState s;
-    __shared__ double sums[8];
-    __shared__ int sh_total, sh_box[6], sh_rebuild, sh_ncand;
-    __shared__ double sh_mass_delta;
-    __shared__ long long sh_dfluid;
-    typedef cub::BlockScan<int, SQ_THREADS> Scan;
-    __shared__ typename Scan::TempStorage scan_tmp;
-
+__device__ __forceinline__ void remap_few(const Lattice& L, const SqArgs& a, SqShared& sh, FewSh& w, int nfew,
+                                          bool corr_step) {
+    SqState& s = sh.s;
     const int tid = threadIdx.x;
-    {   // the state, one word per thread
-        constexpr int NS = (int)(sizeof(SqState) / 4);
-        static_assert(sizeof(SqState) % 4 == 0 && NS <= SQ_THREADS, "one word per thread");
-        if (tid < NS) reinterpret_cast<uint32_t*>(&s)[tid] = reinterpret_cast<const uint32_t*>(a.sq)[tid];
-    }
-    if (tid == 0) {
-        sh_mass_delta = 0.0;
-        sh_dfluid = 0;
+    const int nold = s.n_links;
+#pragma unroll 1
+    for (int k = tid; k < nold; k += SQ_THREADS) w.list[k] = a.links[k];
+    if (tid < nfew) {   // order of the first visit in the box: rank on the visit index
+        const int key = w.fkey[tid];
+        int rank = 0;
+#pragma unroll 1
+        for (int j = 0; j < nfew; ++j) rank += w.fkey[j] < key;
+        w.node[rank] = w.fnode[tid]; w.x[rank] = w.fx[tid]; w.y[rank] = w.fy[tid]; w.z[rank] = w.fz[tid];
+        w.kind[rank] = w.fkind[tid];
     }
     __syncthreads();
-    if (s.status & (ST_NAN | ST_REMAP_RANGE | ST_LINK_OVERFLOW)) return;  // invalid already; the host reports it
-
-    const long long t_now = s.t + 1;
-    const bool loop = (a.stages & STAGE_LOOP) != 0;
-    const bool corr_step = loop && a.corr_step;
-
-    // ---------------- stage BODY ----------------
-    if (a.stages & STAGE_FORCE) {
-        block_sum_rows<6>(a.link_part, s.n_links, LINK_PART, 0, sums);
-        if (tid == 0)
-            for (int d = 0; d < 3; ++d) { s.Fh[d] = sums[d]; s.Th[d] = sums[3 + d]; }
-        __syncthreads();
+    // Everything that is read, in one round: the flags of the changed nodes
+    // and their neighbours, a covered node's populations, an uncovered one's
+    // neighbouring densities ...
+#pragma unroll 1
+    for (int q = tid; q < nfew * Q; q += SQ_THREADS) {
+        const int e = q / Q, j = q - e * Q;
+        const int x = w.x[e], y = w.y[e], z = w.z[e], kind = w.kind[e];
+        const unsigned m = nbr_rt(L, x, y, z, c_cx[j], c_cy[j], c_cz[j]);
+        w.flag[e][j] = a.flag[m];
+        if (kind == 1) w.pop[e][j] = Pop<S>::raw(a.f, logical_slot(L, a.parity, j, w.node[e], x, y, z));
+        else w.nbrho[e][j] = a.rho[m];
+        int o = -1;
+#pragma unroll 1
+        for (int k = 0; k < nfew; ++k)
+            if (w.node[k] == m) o = k;
+        w.nbord[e][j] = o;
+        w.near[e][j] = 0;
     }
-    if (a.stages & STAGE_BODY) {
-        if (tid == 0) {
-            // LBM::applyWallPotential (lbm.cpp:231-241)
-            s.Fw[0] = s.Fw[1] = s.Fw[2] = 0.0;
-            if (L.walls_y) {
-                s.Fw[1] += soft_wall_force(s.X[1] - s.R - 0.5, s.eps, s.FS, s.hc);
-                s.Fw[1] -= soft_wall_force((L.ny - 1.5) - s.X[1] - s.R, s.eps, s.FS, s.hc);
+    __syncthreads();
+    // ... and for each of those nodes whether one of its 18 neighbours is
+    // PARTICLE once the changes are made (a changed node's type follows from
+    // its kind).
+#pragma unroll 1
+    for (int q = tid; q < nfew * Q * 18; q += SQ_THREADS) {
+        const int ej = q / 18, i = q - ej * 18 + 1;
+        const int e = ej / Q, j = ej - e * Q;
+        const int x = wrap1(w.x[e] + c_cx[j], L.nx), y = wrap1(w.y[e] + c_cy[j], L.ny), z = wrap1(w.z[e] + c_cz[j], L.nz);
+        const unsigned m = nbr_rt(L, x, y, z, c_cx[i], c_cy[i], c_cz[i]);
+        bool particle = (a.flag[m] & TYPE_MASK) == T_PARTICLE;
+#pragma unroll 1
+        for (int k = 0; k < nfew; ++k)
+            if (w.node[k] == m) particle = w.kind[k] == 1;
+        if (particle) w.near[e][j] = 1;
+    }
+    if (tid < 32) {   // lane e replays change e; an uncovered node waits for the refills it reads
+        const int e = tid;
+        const bool mine = e < nfew;
+        const int kind = mine ? w.kind[e] : 0;
+        double r[3] = {0, 0, 0}, p[3] = {0, 0, 0};
+        unsigned dep = 0;
+        if (mine) offset_from_squirmer(L, &s, w.x[e], w.y[e], w.z[e], r);
+        if (kind == 1) {   // covered: momentum of the node's populations (lbm.cpp:294-298)
+            double m = 0;
+#pragma unroll 1
+            for (int i = 0; i < Q; ++i) {
+                const double raw = w.pop[e][i];
+                const double fv = S::shifted ? c_w[i] + raw : raw;
+                p[0] += fv * c_cx[i]; p[1] += fv * c_cy[i]; p[2] += fv * c_cz[i];
+                m += raw;
             }
-            if (L.walls_z) {
-                s.Fw[2] += soft_wall_force(s.X[2] - s.R - 0.5, s.eps, s.FS, s.hc);
-                s.Fw[2] -= soft_wall_force((L.nz - 1.5) - s.X[2] - s.R, s.eps, s.FS, s.hc);
+            w.mass[e] = m;
+        } else if (kind == 2) {
+#pragma unroll 1
+            for (int j = 1; j < Q; ++j) {
+                const int o = w.nbord[e][j];
+                if (o >= 0 && o < e && w.kind[o] == 2) dep |= 1u << o;
             }
-            // Squirmer::integrate (squirmer.cpp:52-68)
-            for (int d = 0; d < 3; ++d) {
-                s.U[d] += (s.Fh[d] + s.Fc[d] + s.Fw[d]) / s.M;
-                s.W[d] += (s.Th[d] + s.Tc[d]) / s.I;
-                s.Fc[d] = s.Tc[d] = 0.0;
-            }
-            if (s.planar) { s.U[2] = 0.0; s.W[0] = 0.0; s.W[1] = 0.0; }
-            const double Xold[3] = {s.X[0], s.X[1], s.X[2]};
-            for (int d = 0; d < 3; ++d) s.X[d] += s.U[d];
-            const double we0 = s.W[1] * s.e[2] - s.W[2] * s.e[1];
-            const double we1 = s.W[2] * s.e[0] - s.W[0] * s.e[2];
-            const double we2 = s.W[0] * s.e[1] - s.W[1] * s.e[0];
-            s.e[0] += we0; s.e[1] += we1; s.e[2] += we2;
-            if (s.planar) s.e[2] = 0.0;
-            const double nrm = sqrt(s.e[0] * s.e[0] + s.e[1] * s.e[1] + s.e[2] * s.e[2]);
-            for (int d = 0; d < 3; ++d) s.e[d] /= nrm;
-            // LBM::enforceMinimumGap (lbm.cpp:245-253)
-            for (int d = 1; d <= 2; ++d) {
-                if ((d == 1 && !L.walls_y) || (d == 2 && !L.walls_z)) continue;
-                const int Nd = d == 1 ? L.ny : L.nz;
-                const double lo = 0.5 + s.R + s.hmin, hi = (Nd - 1.5) - s.R - s.hmin;
-                if (s.X[d] < lo) { s.X[d] = lo; if (s.U[d] < 0) s.U[d] = 0; ++s.contacts; }
-                if (s.X[d] > hi) { s.X[d] = hi; if (s.U[d] > 0) s.U[d] = 0; ++s.contacts; }
-            }
-            s.t = t_now;
-            bool ok = true;
-            for (int d = 0; d < 3; ++d)
-                ok = ok && isfinite(s.X[d]) && isfinite(s.U[d]) && isfinite(s.W[d]) && isfinite(s.e[d]) &&
-                     isfinite(s.Fh[d]) && isfinite(s.Th[d]);
-            if (!ok) s.status |= ST_NAN;
-            // The densities the refill reads were stored for the box of the
-            // previous position widened by 2; that covers this step's box
-            // widened by 1 only if the centre moved less than one cell.
-            else if (fabs(s.X[0] - Xold[0]) >= 1.0 || fabs(s.X[1] - Xold[1]) >= 1.0 || fabs(s.X[2] - Xold[2]) >= 1.0)
-                s.status |= ST_REMAP_RANGE;
         }
-        __syncthreads();
-    }
-    if (s.status & (ST_NAN | ST_REMAP_RANGE)) {
-        if (tid == 0) *a.sq = s;
-        return;
-    }
-
-    // the sphere's bounding box (lbm.cpp:272-276)
-    if (tid == 0) {
-        const double R = s.R;
-        int x0 = (int)floor(s.X[0] - R) - 2, x1 = (int)ceil(s.X[0] + R) + 2;
-        int y0 = (int)floor(s.X[1] - R) - 2, y1 = (int)ceil(s.X[1] + R) + 2;
-        int z0 = (int)floor(s.X[2] - R) - 2, z1 = (int)ceil(s.X[2] + R) + 2;
-        if (L.walls_y) { y0 = max(0, y0); y1 = min(L.ny - 1, y1); }
-        sh_box[0] = x0; sh_box[1] = y0; sh_box[2] = z0;
-        sh_box[3] = x1 - x0 + 1; sh_box[4] = y1 - y0 + 1; sh_box[5] = z1 - z0 + 1;
+        bool done = kind != 2;
+#pragma unroll 1
+        for (unsigned all = __ballot_sync(0xffffffffu, done); all != 0xffffffffu;) {
+            if (!done && (dep & ~all) == 0) {   // uncovered: refill (lbm.cpp:302-317)
+                double rs = 0;
+                int cntf = 0;
+#pragma unroll 1
+                for (int j = 1; j < Q; ++j) {
+                    const int o = w.nbord[e][j];
+                    uint8_t ty = w.flag[e][j] & TYPE_MASK;
+                    double rv = w.nbrho[e][j];
+                    if (o >= 0 && o < e) {   // changed earlier
+                        ty = w.kind[o] == 1 ? T_PARTICLE : T_FLUID;
+                        if (w.kind[o] == 2) rv = w.rr[o];
+                    }
+                    if (ty == T_FLUID) { rs += rv; ++cntf; }
+                }
+                const double rr = cntf ? rs / cntf : 1.0;
+                double ub[3];
+                surface_velocity(&s, r, ub, false);
+                w.rr[e] = rr;
+                for (int d = 0; d < 3; ++d) { w.ub[e][d] = ub[d]; p[d] = rr * ub[d]; }
+                const double usq = ub[0] * ub[0] + ub[1] * ub[1] + ub[2] * ub[2];
+#pragma unroll 1
+                for (int i = 0; i < Q; ++i) {   // equilibrium() (lattice.hpp:42-47) at (rr, U + W x r)
+                    const double cu = c_cx[i] * ub[0] + c_cy[i] * ub[1] + c_cz[i] * ub[2];
+                    w.pop[e][i] = c_w[i] * rr * (1.0 + 3.0 * cu + 4.5 * cu * cu - 1.5 * usq);
+                }
+                done = true;
+            }
+            __syncwarp();
+            all = __ballot_sync(0xffffffffu, done);
+        }
+        if (mine) {   // a covered node's momentum is gained, a refilled one's given
+            const double sg = kind == 1 ? 1.0 : -1.0;
+            w.part[e][0] = sg * p[0]; w.part[e][1] = sg * p[1]; w.part[e][2] = sg * p[2];
+            w.part[e][3] = sg * (r[1] * p[2] - r[2] * p[1]);
+            w.part[e][4] = sg * (r[2] * p[0] - r[0] * p[2]);
+            w.part[e][5] = sg * (r[0] * p[1] - r[1] * p[0]);
+        }
+        const unsigned unc = __ballot_sync(0xffffffffu, kind == 2);
+        if (tid < 6) {   // Fc, Tc: the changes in order
+            double* acc = tid < 3 ? &s.Fc[tid] : &s.Tc[tid - 3];
+            double v = *acc;
+#pragma unroll 1
+            for (int k = 0; k < nfew; ++k) v += w.part[k][tid];
+            *acc = v;
+        }
+        if (tid == 0) {
+            sh.nins = sh.nrem = 0;
+            sh.dfluid += 2 * __popc(unc) - nfew;
+            if (corr_step) {
+                double md = sh.mass_delta;
+                for (int k = 0; k < nfew; ++k) {
+                    if (w.kind[k] == 1) md -= w.mass[k];
+                    else
+                        for (int i = 0; i < Q; ++i) md += Pop<S>::stored_raw(w.pop[k][i], i);
+                }
+                sh.mass_delta = md;
+            }
+        }
     }
     __syncthreads();
-    const int bx0 = sh_box[0], by0 = sh_box[1], bz0 = sh_box[2];
-    const int bw = sh_box[3], bh = sh_box[4], bd = sh_box[5];
+    // Scatter: types, refilled populations, rho/u of uncovered nodes; and the
+    // nodes that enter or leave the link list: only the changed nodes and
+    // their neighbours can, each handled once, by the first change it is near.
+#pragma unroll 1
+    for (int q = tid; q < nfew * Q; q += SQ_THREADS) {
+        const int e = q / Q, j = q - e * Q;
+        const unsigned n = w.node[e];
+        if (w.kind[e] == 2) {
+            Pop<S>::put(a.f, logical_slot(L, a.parity, j, n, w.x[e], w.y[e], w.z[e]), j, w.pop[e][j]);
+            if (j == 0) { a.rho[n] = w.rr[e]; a.ux[n] = w.ub[e][0]; a.uy[n] = w.ub[e][1]; a.uz[n] = w.ub[e][2]; }
+        }
+        const int x = wrap1(w.x[e] + c_cx[j], L.nx), y = wrap1(w.y[e] + c_cy[j], L.ny), z = wrap1(w.z[e] + c_cz[j], L.nz);
+        bool first = true;
+#pragma unroll 1
+        for (int k = 0; k < e; ++k) first = first && !near_or_same(L, w, k, x, y, z);
+        if (!first) continue;
+        const unsigned m = (unsigned)x + (unsigned)L.nx * ((unsigned)y + (unsigned)L.ny * (unsigned)z);
+        const int o = w.nbord[e][j];   // the change that m is
+        const uint8_t fm = w.flag[e][j];
+        uint8_t nf = fm & (uint8_t)~NEAR_PARTICLE;
+        if (o >= 0) {
+            const bool nw = (L.walls_y && (y == 1 || y == L.ny - 2)) || (L.walls_z && (z == 1 || z == L.nz - 2));
+            nf = w.kind[o] == 1 ? T_PARTICLE : (uint8_t)(T_FLUID | (nw ? NEAR_WALL : 0));
+        }
+        const bool was = (fm & NEAR_PARTICLE) != 0, is = (nf & TYPE_MASK) == T_FLUID && w.near[e][j];
+        if (is) nf |= NEAR_PARTICLE;
+        if (nf != fm) a.flag[m] = nf;
+        if (is && !was) w.ins[atomicAdd(&sh.nins, 1)] = m;
+        if (was && !is) w.rem[atomicAdd(&sh.nrem, 1)] = m;
+    }
+    __syncthreads();
+    const int nins = sh.nins, nrem = sh.nrem;
+    if (nins + nrem > 0) {   // uniform: every entry to its new place in the ascending list
+#pragma unroll 1
+        for (int k = tid; k < nold + nins; k += SQ_THREADS) {
+            const bool fresh = k >= nold;
+            const unsigned n = fresh ? w.ins[k - nold] : (unsigned)w.list[k];
+            int pos = k;
+            if (fresh) {   // old entries below n
+                int lo = 0, hi = nold;
+#pragma unroll 1
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if ((unsigned)w.list[mid] < n) lo = mid + 1; else hi = mid;
+                }
+                pos = lo;
+            }
+            bool gone = false;
+#pragma unroll 1
+            for (int j = 0; j < nrem; ++j) { pos -= w.rem[j] < n; gone = gone || (!fresh && w.rem[j] == n); }
+#pragma unroll 1
+            for (int j = 0; j < nins; ++j) pos += w.ins[j] < n;
+            if (!gone && pos < a.link_cap && (fresh || pos != k)) {
+                a.links[pos] = (int)n;
+                a.linkslot[n] = pos;
+            }
+        }
+        if (tid == 0) {
+            const int nnew = nold + nins - nrem;
+            s.n_links = min(nnew, a.link_cap);
+            if (nnew > a.link_cap) s.status |= ST_LINK_OVERFLOW;
+        }
+    }
+}
+
+// The remap by the candidate list in full: rebuilds the list where needed,
+// orders any number of changes, and rebuilds the link list by walks over the
+// sphere's box. Off the usual path (remap_few), so it is kept out of line.
+template <class S>
+__device__ __noinline__ void remap_walk(const Lattice& L, const SqArgs& a, SqShared& sh, unsigned char* smem_raw,
+                                        int shell_ok, bool corr_step) {
+    ChgSh* ch = reinterpret_cast<ChgSh*>(smem_raw);
+    typedef cub::BlockScan<int, SQ_THREADS> Scan;
+    SqState& s = sh.s;
+    int &sh_total = sh.total, &sh_rebuild = sh.rebuild, &sh_ncand = sh.ncand;
+    double& sh_mass_delta = sh.mass_delta;
+    long long& sh_dfluid = sh.dfluid;
+    auto& scan_tmp = sh.scan;
+    const int tid = threadIdx.x;
+    const int bx0 = sh.box[0], by0 = sh.box[1], bz0 = sh.box[2];
+    const int bw = sh.box[3], bh = sh.box[4], bd = sh.box[5];
     const int V = bw * bh * bd;
     const double R2 = s.R * s.R;
+    // Wrapped centre for the cheap distance filters (X[0] is kept unwrapped).
+    const double cxw = s.X[0] - L.nx * floor(s.X[0] / L.nx);
+    const double cyw = L.walls_y ? s.X[1] : s.X[1] - L.ny * floor(s.X[1] / L.ny);
+    const double czw = L.walls_z ? s.X[2] : s.X[2] - L.nz * floor(s.X[2] / L.nz);
+    auto approx_r2 = [&](int x, int y, int z) -> double {
+        double dx = x - cxw, dy = y - cyw, dz = z - czw;
+        if (dx > 0.5 * L.nx) dx -= L.nx; else if (dx < -0.5 * L.nx) dx += L.nx;
+        if (!L.walls_y) { if (dy > 0.5 * L.ny) dy -= L.ny; else if (dy < -0.5 * L.ny) dy += L.ny; }
+        if (!L.walls_z) { if (dz > 0.5 * L.nz) dz -= L.nz; else if (dz < -0.5 * L.nz) dz += L.nz; }
+        return dx * dx + dy * dy + dz * dz;
+    };
+    // Only nodes within one cell of the sphere's surface can change: the
+    // centre moved less than a cell since the last remap (checked in stage
+    // BODY), so nodes deeper than that were and stay PARTICLE and nodes
+    // farther out were and stay FLUID. The candidates are the nodes within
+    // R +- 1.05 of the centre (0.05 covers the cheap distance against the
+    // reference's exact offset, which makes the decision). The shell list
+    // widens that by SHELL_SLACK around a reference centre, so it holds
+    // every candidate while the centre stays within SHELL_SLACK of it
+    // (triangle inequality), and the box walk that builds it runs only
+    // when the centre leaves that ball.
 
-    // ---------------- stage REMAP ----------------
-    if (a.stages & STAGE_REMAP) {
-        // Wrapped centre for the cheap distance filters (X[0] is kept unwrapped).
-        const double cxw = s.X[0] - L.nx * floor(s.X[0] / L.nx);
-        const double cyw = L.walls_y ? s.X[1] : s.X[1] - L.ny * floor(s.X[1] / L.ny);
-        const double czw = L.walls_z ? s.X[2] : s.X[2] - L.nz * floor(s.X[2] / L.nz);
-        auto approx_r2 = [&](int x, int y, int z) -> double {
-            double dx = x - cxw, dy = y - cyw, dz = z - czw;
-            if (dx > 0.5 * L.nx) dx -= L.nx; else if (dx < -0.5 * L.nx) dx += L.nx;
-            if (!L.walls_y) { if (dy > 0.5 * L.ny) dy -= L.ny; else if (dy < -0.5 * L.ny) dy += L.ny; }
-            if (!L.walls_z) { if (dz > 0.5 * L.nz) dz -= L.nz; else if (dz < -0.5 * L.nz) dz += L.nz; }
-            return dx * dx + dy * dy + dz * dz;
-        };
-        // Only nodes within one cell of the sphere's surface can change: the
-        // centre moved less than a cell since the last remap (checked in stage
-        // BODY), so nodes deeper than that were and stay PARTICLE and nodes
-        // farther out were and stay FLUID. The candidates are the nodes within
-        // R +- 1.05 of the centre (0.05 covers the cheap distance against the
-        // reference's exact offset, which makes the decision). The shell list
-        // widens that by SHELL_SLACK around a reference centre, so it holds
-        // every candidate while the centre stays within SHELL_SLACK of it
-        // (triangle inequality), and the box walk that builds it runs only
-        // when the centre leaves that ball.
-
-        // (1) candidates: the cached shell, rebuilt in box order (z, y, x of
-        // the first visit) when the centre has left the slack around the
-        // reference centre of the list. A cached list that yields more than
-        // SQ_SORT_CAP changes is rebuilt at once (second pass).
-        if (tid == 0) {
-            const ShellCache hc = *a.shell_hdr;
-            const double d0 = s.X[0] - hc.X[0], d1 = s.X[1] - hc.X[1], d2 = s.X[2] - hc.X[2];
-            sh_rebuild = !(hc.valid && d0 * d0 + d1 * d1 + d2 * d2 < SHELL_SLACK * SHELL_SLACK);
-            sh_ncand = hc.n;
-        }
-        __syncthreads();
-        for (int pass = 0; pass < 2; ++pass) {
-            if (pass == 1) {
-                if (!(!sh_rebuild && sh_total > SQ_SORT_CAP)) break;   // uniform
-                __syncthreads();
-                if (tid == 0) sh_rebuild = 1;
-                __syncthreads();
-            }
-            const int chunk = (V + SQ_THREADS - 1) / SQ_THREADS;
-            const int k0 = min(V, tid * chunk), k1 = min(V, k0 + chunk);
-            auto box_walk = [&](auto&& visit) {
-                if (k0 >= k1) return;
-                int bx = k0 % bw, by = (k0 / bw) % bh, bz = k0 / (bw * bh);
-                int x = (((bx0 + bx) % L.nx) + L.nx) % L.nx;
-                int y = (((by0 + by) % L.ny) + L.ny) % L.ny;
-                int z = (((bz0 + bz) % L.nz) + L.nz) % L.nz;
-                for (int k = k0; k < k1; ++k) {
-                    // a box wider than the lattice revisits nodes; the first visit counts
-                    if (bx < L.nx && by < L.ny && bz < L.nz) visit(k, x, y, z);
-                    if (++bx == bw) {
-                        bx = 0; x = (((bx0) % L.nx) + L.nx) % L.nx;
-                        if (++by == bh) { by = 0; y = (((by0) % L.ny) + L.ny) % L.ny; ++bz; if (++z == L.nz) z = 0; }
-                        else if (++y == L.ny) y = 0;
-                    } else if (++x == L.nx) x = 0;
-                }
-            };
-            if (sh_rebuild) {   // uniform
-                const double Sin = fmax(s.R - 1.05 - SHELL_SLACK, 0.0), Sout = s.R + 1.05 + SHELL_SLACK;
-                const double Sin2 = Sin * Sin, Sout2 = Sout * Sout;
-                int cnt = 0;
-                box_walk([&](int, int x, int y, int z) {
-                    const double r2 = approx_r2(x, y, z);
-                    cnt += (r2 >= Sin2 && r2 < Sout2);
-                });
-                int off = 0;
-                Scan(scan_tmp).ExclusiveSum(cnt, off, sh_total);
-                __syncthreads();
-                box_walk([&](int, int x, int y, int z) {
-                    const double r2 = approx_r2(x, y, z);
-                    if (r2 >= Sin2 && r2 < Sout2) {
-                        if (off < a.chg_cap) a.shell[off] = x + L.nx * (y + L.ny * z);
-                        ++off;
-                    }
-                });
-                if (tid == 0) {
-                    sh_ncand = min(sh_total, a.chg_cap);
-                    ShellCache hc;
-                    for (int d = 0; d < 3; ++d) hc.X[d] = s.X[d];
-                    hc.n = sh_ncand;
-                    hc.valid = 1;
-                    *a.shell_hdr = hc;
-                }
-                __syncthreads();
-            }
-            const int ncand = sh_ncand;
-            // (2) exact test of each candidate (flag load + the reference's
-            // offset), SQ_GROUP candidates per thread at a time: their node
-            // indices and flags are all loaded before the first test
-            for (int c0 = tid; c0 < ncand; c0 += SQ_GROUP * SQ_THREADS) {
-                unsigned nn[SQ_GROUP];
-                uint8_t ty[SQ_GROUP];
-#pragma unroll
-                for (int g = 0; g < SQ_GROUP; ++g) {
-                    const int c = c0 + g * SQ_THREADS;
-                    nn[g] = c < ncand ? (unsigned)a.shell[c] : 0u;
-                }
-#pragma unroll
-                for (int g = 0; g < SQ_GROUP; ++g)
-                    ty[g] = c0 + g * SQ_THREADS < ncand ? (uint8_t)(a.flag[nn[g]] & TYPE_MASK) : (uint8_t)T_WALL;
-#pragma unroll
-                for (int g = 0; g < SQ_GROUP; ++g) {
-                    const int c = c0 + g * SQ_THREADS;
-                    if (c >= ncand) break;
-                    const unsigned n = nn[g];
-                    uint8_t mk = 0;
-                    if (ty[g] != T_WALL) {
-                        const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
-                                  z = (int)(n / L.nxy);
-                        double r[3];
-                        offset_from_squirmer(L, &s, x, y, z, r);
-                        const bool inside = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] < R2;
-                        if (inside != (ty[g] == T_PARTICLE)) mk = inside ? 1 : 2;
-                    }
-                    a.mark[c] = mk;
-                }
-            }
+    // (1) candidates: the cached shell, rebuilt in box order (z, y, x of
+    // the first visit) when the centre has left the slack around the
+    // reference centre of the list. A cached list that yields more than
+    // SQ_SORT_CAP changes is rebuilt at once (second pass).
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass == 1) {
+            if (!(!sh_rebuild && sh_total > SQ_SORT_CAP)) break;   // uniform
             __syncthreads();
-            // (3) changed nodes in list order
-            {
-                const int ch2 = (ncand + SQ_THREADS - 1) / SQ_THREADS;
-                const int c0 = min(ncand, tid * ch2), c1 = min(ncand, c0 + ch2);
-                int cnt = 0;
-                for (int c = c0; c < c1; ++c) cnt += a.mark[c] != 0;
-                int off = 0;
-                Scan(scan_tmp).ExclusiveSum(cnt, off, sh_total);
-                __syncthreads();
-                for (int c = c0; c < c1; ++c) {
-                    const uint8_t mk = a.mark[c];
-                    if (!mk) continue;
-                    a.chg_node[off] = a.shell[c];
-                    a.chg_key[off] = mk;
+            if (tid == 0) sh_rebuild = 1;
+            __syncthreads();
+        }
+        const int chunk = (V + SQ_THREADS - 1) / SQ_THREADS;
+        const int k0 = min(V, tid * chunk), k1 = min(V, k0 + chunk);
+        auto box_walk = [&](auto&& visit) {
+            if (k0 >= k1) return;
+            int bx = k0 % bw, by = (k0 / bw) % bh, bz = k0 / (bw * bh);
+            int x = (((bx0 + bx) % L.nx) + L.nx) % L.nx;
+            int y = (((by0 + by) % L.ny) + L.ny) % L.ny;
+            int z = (((bz0 + bz) % L.nz) + L.nz) % L.nz;
+            for (int k = k0; k < k1; ++k) {
+                // a box wider than the lattice revisits nodes; the first visit counts
+                if (bx < L.nx && by < L.ny && bz < L.nz) visit(k, x, y, z);
+                if (++bx == bw) {
+                    bx = 0; x = (((bx0) % L.nx) + L.nx) % L.nx;
+                    if (++by == bh) { by = 0; y = (((by0) % L.ny) + L.ny) % L.ny; ++bz; if (++z == L.nz) z = 0; }
+                    else if (++y == L.ny) y = 0;
+                } else if (++x == L.nx) x = 0;
+            }
+        };
+        if (sh_rebuild) {   // uniform
+            const double Sin = fmax(s.R - 1.05 - SHELL_SLACK, 0.0), Sout = s.R + 1.05 + SHELL_SLACK;
+            const double Sin2 = Sin * Sin, Sout2 = Sout * Sout;
+            int cnt = 0;
+            box_walk([&](int, int x, int y, int z) {
+                const double r2 = approx_r2(x, y, z);
+                cnt += (r2 >= Sin2 && r2 < Sout2);
+            });
+            int off = 0;
+            Scan(scan_tmp).ExclusiveSum(cnt, off, sh_total);
+            __syncthreads();
+            box_walk([&](int, int x, int y, int z) {
+                const double r2 = approx_r2(x, y, z);
+                if (r2 >= Sin2 && r2 < Sout2) {
+                    if (off < a.chg_cap) a.shell[off] = x + L.nx * (y + L.ny * z);
                     ++off;
                 }
-            }
-            __syncthreads();
-        }
-        // A list cached under an earlier box is in that box's order: put the
-        // changes in the order of their first visit in this box (rank sort on
-        // the visit index; distinct nodes have distinct indices).
-        if (!sh_rebuild && sh_total > 1) {   // uniform
-            const int nchg = sh_total;
-            int* keys = reinterpret_cast<int*>(smem_raw);
-            int* nodes = keys + SQ_SORT_CAP;
-            int* kinds = nodes + SQ_SORT_CAP;
-            for (int e = tid; e < nchg; e += SQ_THREADS) {
-                const unsigned n = (unsigned)a.chg_node[e];
-                const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
-                          z = (int)(n / L.nxy);
-                const int kx = ((x - bx0) % L.nx + L.nx) % L.nx;
-                const int ky = ((y - by0) % L.ny + L.ny) % L.ny;
-                const int kz = ((z - bz0) % L.nz + L.nz) % L.nz;
-                keys[e] = (kz * bh + ky) * bw + kx;
-                nodes[e] = (int)n;
-                kinds[e] = a.chg_key[e];
-            }
-            __syncthreads();
-            for (int e = tid; e < nchg; e += SQ_THREADS) {
-                const int ke = keys[e];
-                int rank = 0;
-                for (int j = 0; j < nchg; ++j) rank += keys[j] < ke;
-                a.chg_node[rank] = nodes[e];
-                a.chg_key[rank] = kinds[e];
-            }
-            __syncthreads();
-        }
-        const int total = sh_total;
-        for (int k = tid; k < total; k += SQ_THREADS) a.ordermap[a.chg_node[k]] = k;
-        __syncthreads();
-
-        // (4) batches: gather, ordered replay, scatter
-        for (int b0 = 0; b0 < total; b0 += SQ_BATCH) {
-            const int nb = min(SQ_BATCH, total - b0);
-            for (int e = tid; e < nb; e += SQ_THREADS) {
-                ChgSh& c = ch[e];
-                const unsigned n = (unsigned)a.chg_node[b0 + e];
-                c.node = (int)n;
-                c.kind = a.chg_key[b0 + e];
-                const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
-                          z = (int)(n / L.nxy);
-                offset_from_squirmer(L, &s, x, y, z, c.r);
-                if (c.kind == 1) {
-                    // covered: momentum of the node's populations (lbm.cpp:294-298)
-                    double p0 = 0, p1 = 0, p2 = 0, m = 0;
-                    for (int i = 0; i < Q; ++i) {
-                        const size_t k = logical_slot(L, a.parity, i, n, x, y, z);
-                        const double fv = Pop<S>::get(a.f, k, i);
-                        p0 += fv * c_cx[i]; p1 += fv * c_cy[i]; p2 += fv * c_cz[i];
-                        m += Pop<S>::raw(a.f, k);
-                    }
-                    c.p[0] = p0; c.p[1] = p1; c.p[2] = p2; c.mass = m;
-                }
-            }
-            __syncthreads();
-            for (int q = tid; q < nb * 18; q += SQ_THREADS) {
-                const int e = q / 18, j = q % 18 + 1;
-                ChgSh& c = ch[e];
-                if (c.kind != 2) continue;
-                const unsigned n = (unsigned)c.node;
-                const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
-                          z = (int)(n / L.nxy);
-                // lbm.cpp:305: neighbour with wrap in every axis
-                const int xn = (x + c_cx[j] + L.nx) % L.nx, yn = (y + c_cy[j] + L.ny) % L.ny,
-                          zn = (z + c_cz[j] + L.nz) % L.nz;
-                const unsigned m = (unsigned)xn + (unsigned)L.nx * ((unsigned)yn + (unsigned)L.ny * (unsigned)zn);
-                c.nbfl[j - 1] = a.flag[m] & TYPE_MASK;
-                c.nbrho[j - 1] = a.rho[m];
-                c.nbord[j - 1] = a.ordermap[m];
-            }
-            __syncthreads();
+            });
             if (tid == 0) {
-                for (int e = 0; e < nb; ++e) {
-                    ChgSh& c = ch[e];
-                    if (c.kind == 1) {
-                        const double t0 = c.r[1] * c.p[2] - c.r[2] * c.p[1];
-                        const double t1 = c.r[2] * c.p[0] - c.r[0] * c.p[2];
-                        const double t2 = c.r[0] * c.p[1] - c.r[1] * c.p[0];
-                        s.Fc[0] += c.p[0]; s.Tc[0] += t0;
-                        s.Fc[1] += c.p[1]; s.Tc[1] += t1;
-                        s.Fc[2] += c.p[2]; s.Tc[2] += t2;
-                        if (corr_step) sh_mass_delta -= c.mass;
-                        sh_dfluid -= 1;
-                        continue;
-                    }
-                    // uncovered: refill (lbm.cpp:302-317)
-                    double rs = 0; int cntf = 0;
-                    const int k_me = b0 + e;
-                    for (int j = 0; j < 18; ++j) {
-                        const int o = c.nbord[j];
-                        uint8_t ty = c.nbfl[j];
-                        double rv = c.nbrho[j];
-                        if (o >= b0 && o < k_me) {  // changed earlier in this batch
-                            const ChgSh& cc = ch[o - b0];
-                            ty = cc.kind == 1 ? T_PARTICLE : T_FLUID;
-                            if (cc.kind == 2) rv = cc.rr;
-                        }
-                        if (ty == T_FLUID) { rs += rv; ++cntf; }
-                    }
-                    const double rr = cntf ? rs / cntf : 1.0;
-                    double ub[3];
-                    surface_velocity(&s, c.r, ub, false);
-                    c.rr = rr; c.ub[0] = ub[0]; c.ub[1] = ub[1]; c.ub[2] = ub[2];
-                    const double p0 = rr * ub[0], p1 = rr * ub[1], p2 = rr * ub[2];
-                    const double t0 = c.r[1] * p2 - c.r[2] * p1;
-                    const double t1 = c.r[2] * p0 - c.r[0] * p2;
-                    const double t2 = c.r[0] * p1 - c.r[1] * p0;
-                    s.Fc[0] -= p0; s.Tc[0] -= t0;
-                    s.Fc[1] -= p1; s.Tc[1] -= t1;
-                    s.Fc[2] -= p2; s.Tc[2] -= t2;
-                    sh_dfluid += 1;
-                    if (corr_step) {
-                        const double usq = ub[0] * ub[0] + ub[1] * ub[1] + ub[2] * ub[2];
-                        for (int i = 0; i < Q; ++i) {
-                            const double cu = c_cx[i] * ub[0] + c_cy[i] * ub[1] + c_cz[i] * ub[2];
-                            const double feq = c_w[i] * rr * (1.0 + 3.0 * cu + 4.5 * cu * cu - 1.5 * usq);
-                            sh_mass_delta += Pop<S>::stored_raw(feq, i);
-                        }
-                    }
-                }
-            }
-            __syncthreads();
-            // scatter: flags, refilled populations, rho/u of uncovered nodes
-            for (int q = tid; q < nb * Q; q += SQ_THREADS) {
-                const int e = q / Q, i = q % Q;
-                const ChgSh& c = ch[e];
-                const unsigned n = (unsigned)c.node;
-                const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
-                          z = (int)(n / L.nxy);
-                if (i == 0) {
-                    uint8_t nf = T_PARTICLE;
-                    if (c.kind == 2) {
-                        const bool nw = (L.walls_y && (y == 1 || y == L.ny - 2)) || (L.walls_z && (z == 1 || z == L.nz - 2));
-                        nf = T_FLUID | (nw ? NEAR_WALL : 0);
-                        a.rho[n] = c.rr; a.ux[n] = c.ub[0]; a.uy[n] = c.ub[1]; a.uz[n] = c.ub[2];
-                    }
-                    a.flag[n] = nf;
-                }
-                if (c.kind == 2) {
-                    // equilibrium() (lattice.hpp:42-47) at (rr, U + W x r)
-                    const double cu = c_cx[i] * c.ub[0] + c_cy[i] * c.ub[1] + c_cz[i] * c.ub[2];
-                    const double usq = c.ub[0] * c.ub[0] + c.ub[1] * c.ub[1] + c.ub[2] * c.ub[2];
-                    const double feq = c_w[i] * c.rr * (1.0 + 3.0 * cu + 4.5 * cu * cu - 1.5 * usq);
-                    Pop<S>::put(a.f, logical_slot(L, a.parity, i, n, x, y, z), i, feq);
-                }
+                sh_ncand = min(sh_total, a.chg_cap);
+                ShellCache hc;
+                for (int d = 0; d < 3; ++d) hc.X[d] = s.X[d];
+                hc.n = sh_ncand;
+                hc.valid = shell_ok == 2 ? 2 : 1;
+                *a.shell_hdr = hc;
             }
             __syncthreads();
         }
-        for (int k = tid; k < total; k += SQ_THREADS) a.ordermap[a.chg_node[k]] = -1;
-
-        // (5) boundary-link list: FLUID nodes with a PARTICLE neighbour, in
-        // ascending node order over the sphere's box.
-        if (total > 0 || s.n_links < 0) {
-            const int old = max(0, s.n_links);
-            for (int k = tid; k < old; k += SQ_THREADS) {
-                const int n = a.links[k];
-                a.flag[n] &= (uint8_t)~NEAR_PARTICLE;
+        const int ncand = sh_ncand;
+        // (2) exact test of each candidate (flag load + the reference's
+        // offset), SQ_GROUP candidates per thread at a time: their node
+        // indices and flags are all loaded before the first test
+        for (int c0 = tid; c0 < ncand; c0 += SQ_GROUP * SQ_THREADS) {
+            unsigned nn[SQ_GROUP];
+            uint8_t ty[SQ_GROUP];
+#pragma unroll
+            for (int g = 0; g < SQ_GROUP; ++g) {
+                const int c = c0 + g * SQ_THREADS;
+                nn[g] = c < ncand ? (unsigned)a.shell[c] : 0u;
             }
-            __syncthreads();
-            AxisRange ax, ay, az;
-            ax.init(bx0, bw, L.nx); ay.init(by0, bh, L.ny); az.init(bz0, bd, L.nz);
-            const int V2 = ax.width * ay.width * az.width;
-            // after the remap FLUID means r >= R; PARTICLE neighbours lie within sqrt(2)
-            const double Lin = fmax(s.R - 0.05, 0.0), Lout = s.R + 1.5;
-            const double Lin2 = Lin * Lin, Lout2 = Lout * Lout;
-            const int chk = (V2 + SQ_THREADS - 1) / SQ_THREADS;
-            const int q0 = min(V2, tid * chk), q1 = min(V2, q0 + chk);
-            auto region_walk = [&](auto&& visit) {
-                for (int k = q0; k < q1; ++k) {
-                    const int x = ax.at(k % ax.width), y = ay.at((k / ax.width) % ay.width),
-                              z = az.at(k / (ax.width * ay.width));
-                    visit(x, y, z);
-                }
-            };
-            {
-                int cnt = 0;
-                region_walk([&](int x, int y, int z) {
-                    const double r2 = approx_r2(x, y, z);
-                    cnt += (r2 >= Lin2 && r2 < Lout2);
-                });
-                int off = 0;
-                Scan(scan_tmp).ExclusiveSum(cnt, off, sh_total);
-                __syncthreads();
-                region_walk([&](int x, int y, int z) {
-                    const double r2 = approx_r2(x, y, z);
-                    if (r2 >= Lin2 && r2 < Lout2) {
-                        if (off < a.chg_cap) a.cand[off] = x + L.nx * (y + L.ny * z);
-                        ++off;
-                    }
-                });
-            }
-            __syncthreads();
-            const int nc2 = min(sh_total, a.chg_cap);
-            for (int c = tid; c < nc2; c += SQ_THREADS) {
-                const unsigned n = (unsigned)a.cand[c];
+#pragma unroll
+            for (int g = 0; g < SQ_GROUP; ++g)
+                ty[g] = c0 + g * SQ_THREADS < ncand ? (uint8_t)(a.flag[nn[g]] & TYPE_MASK) : (uint8_t)T_WALL;
+#pragma unroll
+            for (int g = 0; g < SQ_GROUP; ++g) {
+                const int c = c0 + g * SQ_THREADS;
+                if (c >= ncand) break;
+                const unsigned n = nn[g];
                 uint8_t mk = 0;
-                if ((a.flag[n] & TYPE_MASK) == T_FLUID) {
+                if (ty[g] != T_WALL) {
                     const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
                               z = (int)(n / L.nxy);
-                    const Nbr nbh(L, x, y, z);
-                    bool near = false;
-#pragma unroll
-                    for (int j = 1; j < Q; ++j) near |= (a.flag[nbh.of(n, j)] & TYPE_MASK) == T_PARTICLE;
-                    mk = near;
+                    double r[3];
+                    offset_from_squirmer(L, &s, x, y, z, r);
+                    const bool inside = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] < R2;
+                    if (inside != (ty[g] == T_PARTICLE)) mk = inside ? 1 : 2;
                 }
                 a.mark[c] = mk;
             }
+        }
+        __syncthreads();
+        // (3) changed nodes in list order
+        {
+            const int ch2 = (ncand + SQ_THREADS - 1) / SQ_THREADS;
+            const int c0 = min(ncand, tid * ch2), c1 = min(ncand, c0 + ch2);
+            int cnt = 0;
+            for (int c = c0; c < c1; ++c) cnt += a.mark[c] != 0;
+            int off = 0;
+            Scan(scan_tmp).ExclusiveSum(cnt, off, sh_total);
             __syncthreads();
-            {
-                const int ch2 = (nc2 + SQ_THREADS - 1) / SQ_THREADS;
-                const int c0 = min(nc2, tid * ch2), c1 = min(nc2, c0 + ch2);
-                int cnt = 0;
-                for (int c = c0; c < c1; ++c) cnt += a.mark[c];
-                int off = 0;
-                Scan(scan_tmp).ExclusiveSum(cnt, off, sh_total);
-                __syncthreads();
-                for (int c = c0; c < c1; ++c) {
-                    if (!a.mark[c]) continue;
-                    const int n = a.cand[c];
-                    if (off < a.link_cap) {
-                        a.links[off] = n;
-                        a.linkslot[n] = off;
-                        a.flag[n] |= NEAR_PARTICLE;
-                    }
-                    ++off;
-                }
-            }
-            __syncthreads();
-            if (tid == 0) {
-                s.n_links = min(sh_total, a.link_cap);
-                if (sh_total > a.link_cap) s.status |= ST_LINK_OVERFLOW;
+            for (int c = c0; c < c1; ++c) {
+                const uint8_t mk = a.mark[c];
+                if (!mk) continue;
+                a.chg_node[off] = a.shell[c];
+                a.chg_key[off] = mk;
+                ++off;
             }
         }
-        if (tid == 0) s.n_fluid += sh_dfluid;
+        __syncthreads();
+    }
+    // A list cached under an earlier box is in that box's order: put the
+    // changes in the order of their first visit in this box (rank sort on
+    // the visit index; distinct nodes have distinct indices).
+    if (!sh_rebuild && sh_total > 1) {   // uniform
+        const int nchg = sh_total;
+        int* keys = reinterpret_cast<int*>(smem_raw);
+        int* nodes = keys + SQ_SORT_CAP;
+        int* kinds = nodes + SQ_SORT_CAP;
+        for (int e = tid; e < nchg; e += SQ_THREADS) {
+            const unsigned n = (unsigned)a.chg_node[e];
+            const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
+                      z = (int)(n / L.nxy);
+            const int kx = ((x - bx0) % L.nx + L.nx) % L.nx;
+            const int ky = ((y - by0) % L.ny + L.ny) % L.ny;
+            const int kz = ((z - bz0) % L.nz + L.nz) % L.nz;
+            keys[e] = (kz * bh + ky) * bw + kx;
+            nodes[e] = (int)n;
+            kinds[e] = a.chg_key[e];
+        }
+        __syncthreads();
+        for (int e = tid; e < nchg; e += SQ_THREADS) {
+            const int ke = keys[e];
+            int rank = 0;
+            for (int j = 0; j < nchg; ++j) rank += keys[j] < ke;
+            a.chg_node[rank] = nodes[e];
+            a.chg_key[rank] = kinds[e];
+        }
+        __syncthreads();
+    }
+    const int total = sh_total;
+    for (int k = tid; k < total; k += SQ_THREADS) a.ordermap[a.chg_node[k]] = k;
+    __syncthreads();
+
+    // (4) batches: gather, ordered replay, scatter
+    for (int b0 = 0; b0 < total; b0 += SQ_BATCH) {
+        const int nb = min(SQ_BATCH, total - b0);
+        for (int e = tid; e < nb; e += SQ_THREADS) {
+            ChgSh& c = ch[e];
+            const unsigned n = (unsigned)a.chg_node[b0 + e];
+            c.node = (int)n;
+            c.kind = a.chg_key[b0 + e];
+            const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
+                      z = (int)(n / L.nxy);
+            offset_from_squirmer(L, &s, x, y, z, c.r);
+            if (c.kind == 1) {
+                // covered: momentum of the node's populations (lbm.cpp:294-298)
+                double p0 = 0, p1 = 0, p2 = 0, m = 0;
+                for (int i = 0; i < Q; ++i) {
+                    const size_t k = logical_slot(L, a.parity, i, n, x, y, z);
+                    const double fv = Pop<S>::get(a.f, k, i);
+                    p0 += fv * c_cx[i]; p1 += fv * c_cy[i]; p2 += fv * c_cz[i];
+                    m += Pop<S>::raw(a.f, k);
+                }
+                c.p[0] = p0; c.p[1] = p1; c.p[2] = p2; c.mass = m;
+            }
+        }
+        __syncthreads();
+        for (int q = tid; q < nb * 18; q += SQ_THREADS) {
+            const int e = q / 18, j = q % 18 + 1;
+            ChgSh& c = ch[e];
+            if (c.kind != 2) continue;
+            const unsigned n = (unsigned)c.node;
+            const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
+                      z = (int)(n / L.nxy);
+            // lbm.cpp:305: neighbour with wrap in every axis
+            const int xn = (x + c_cx[j] + L.nx) % L.nx, yn = (y + c_cy[j] + L.ny) % L.ny,
+                      zn = (z + c_cz[j] + L.nz) % L.nz;
+            const unsigned m = (unsigned)xn + (unsigned)L.nx * ((unsigned)yn + (unsigned)L.ny * (unsigned)zn);
+            c.nbfl[j - 1] = a.flag[m] & TYPE_MASK;
+            c.nbrho[j - 1] = a.rho[m];
+            c.nbord[j - 1] = a.ordermap[m];
+        }
+        __syncthreads();
+        if (tid == 0) {
+            for (int e = 0; e < nb; ++e) {
+                ChgSh& c = ch[e];
+                if (c.kind == 1) {
+                    const double t0 = c.r[1] * c.p[2] - c.r[2] * c.p[1];
+                    const double t1 = c.r[2] * c.p[0] - c.r[0] * c.p[2];
+                    const double t2 = c.r[0] * c.p[1] - c.r[1] * c.p[0];
+                    s.Fc[0] += c.p[0]; s.Tc[0] += t0;
+                    s.Fc[1] += c.p[1]; s.Tc[1] += t1;
+                    s.Fc[2] += c.p[2]; s.Tc[2] += t2;
+                    if (corr_step) sh_mass_delta -= c.mass;
+                    sh_dfluid -= 1;
+                    continue;
+                }
+                // uncovered: refill (lbm.cpp:302-317)
+                double rs = 0; int cntf = 0;
+                const int k_me = b0 + e;
+                for (int j = 0; j < 18; ++j) {
+                    const int o = c.nbord[j];
+                    uint8_t ty = c.nbfl[j];
+                    double rv = c.nbrho[j];
+                    if (o >= b0 && o < k_me) {  // changed earlier in this batch
+                        const ChgSh& cc = ch[o - b0];
+                        ty = cc.kind == 1 ? T_PARTICLE : T_FLUID;
+                        if (cc.kind == 2) rv = cc.rr;
+                    }
+                    if (ty == T_FLUID) { rs += rv; ++cntf; }
+                }
+                const double rr = cntf ? rs / cntf : 1.0;
+                double ub[3];
+                surface_velocity(&s, c.r, ub, false);
+                c.rr = rr; c.ub[0] = ub[0]; c.ub[1] = ub[1]; c.ub[2] = ub[2];
+                const double p0 = rr * ub[0], p1 = rr * ub[1], p2 = rr * ub[2];
+                const double t0 = c.r[1] * p2 - c.r[2] * p1;
+                const double t1 = c.r[2] * p0 - c.r[0] * p2;
+                const double t2 = c.r[0] * p1 - c.r[1] * p0;
+                s.Fc[0] -= p0; s.Tc[0] -= t0;
+                s.Fc[1] -= p1; s.Tc[1] -= t1;
+                s.Fc[2] -= p2; s.Tc[2] -= t2;
+                sh_dfluid += 1;
+                if (corr_step) {
+                    const double usq = ub[0] * ub[0] + ub[1] * ub[1] + ub[2] * ub[2];
+                    for (int i = 0; i < Q; ++i) {
+                        const double cu = c_cx[i] * ub[0] + c_cy[i] * ub[1] + c_cz[i] * ub[2];
+                        const double feq = c_w[i] * rr * (1.0 + 3.0 * cu + 4.5 * cu * cu - 1.5 * usq);
+                        sh_mass_delta += Pop<S>::stored_raw(feq, i);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        // scatter: flags, refilled populations, rho/u of uncovered nodes
+        for (int q = tid; q < nb * Q; q += SQ_THREADS) {
+            const int e = q / Q, i = q % Q;
+            const ChgSh& c = ch[e];
+            const unsigned n = (unsigned)c.node;
+            const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
+                      z = (int)(n / L.nxy);
+            if (i == 0) {
+                uint8_t nf = T_PARTICLE;
+                if (c.kind == 2) {
+                    const bool nw = (L.walls_y && (y == 1 || y == L.ny - 2)) || (L.walls_z && (z == 1 || z == L.nz - 2));
+                    nf = T_FLUID | (nw ? NEAR_WALL : 0);
+                    a.rho[n] = c.rr; a.ux[n] = c.ub[0]; a.uy[n] = c.ub[1]; a.uz[n] = c.ub[2];
+                }
+                a.flag[n] = nf;
+            }
+            if (c.kind == 2) {
+                // equilibrium() (lattice.hpp:42-47) at (rr, U + W x r)
+                const double cu = c_cx[i] * c.ub[0] + c_cy[i] * c.ub[1] + c_cz[i] * c.ub[2];
+                const double usq = c.ub[0] * c.ub[0] + c.ub[1] * c.ub[1] + c.ub[2] * c.ub[2];
+                const double feq = c_w[i] * c.rr * (1.0 + 3.0 * cu + 4.5 * cu * cu - 1.5 * usq);
+                Pop<S>::put(a.f, logical_slot(L, a.parity, i, n, x, y, z), i, feq);
+            }
+        }
+        __syncthreads();
+    }
+    for (int k = tid; k < total; k += SQ_THREADS) a.ordermap[a.chg_node[k]] = -1;
+
+    // (5) boundary-link list: FLUID nodes with a PARTICLE neighbour, in
+    // ascending node order over the sphere's box.
+    if (total > 0 || s.n_links < 0) {
+        const int old = max(0, s.n_links);
+        for (int k = tid; k < old; k += SQ_THREADS) {
+            const int n = a.links[k];
+            a.flag[n] &= (uint8_t)~NEAR_PARTICLE;
+        }
+        __syncthreads();
+        AxisRange ax, ay, az;
+        ax.init(bx0, bw, L.nx); ay.init(by0, bh, L.ny); az.init(bz0, bd, L.nz);
+        const int V2 = ax.width * ay.width * az.width;
+        // after the remap FLUID means r >= R; PARTICLE neighbours lie within sqrt(2)
+        const double Lin = fmax(s.R - 0.05, 0.0), Lout = s.R + 1.5;
+        const double Lin2 = Lin * Lin, Lout2 = Lout * Lout;
+        const int chk = (V2 + SQ_THREADS - 1) / SQ_THREADS;
+        const int q0 = min(V2, tid * chk), q1 = min(V2, q0 + chk);
+        auto region_walk = [&](auto&& visit) {
+            for (int k = q0; k < q1; ++k) {
+                const int x = ax.at(k % ax.width), y = ay.at((k / ax.width) % ay.width),
+                          z = az.at(k / (ax.width * ay.width));
+                visit(x, y, z);
+            }
+        };
+        {
+            int cnt = 0;
+            region_walk([&](int x, int y, int z) {
+                const double r2 = approx_r2(x, y, z);
+                cnt += (r2 >= Lin2 && r2 < Lout2);
+            });
+            int off = 0;
+            Scan(scan_tmp).ExclusiveSum(cnt, off, sh_total);
+            __syncthreads();
+            region_walk([&](int x, int y, int z) {
+                const double r2 = approx_r2(x, y, z);
+                if (r2 >= Lin2 && r2 < Lout2) {
+                    if (off < a.chg_cap) a.cand[off] = x + L.nx * (y + L.ny * z);
+                    ++off;
+                }
+            });
+        }
+        __syncthreads();
+        const int nc2 = min(sh_total, a.chg_cap);
+        for (int c = tid; c < nc2; c += SQ_THREADS) {
+            const unsigned n = (unsigned)a.cand[c];
+            uint8_t mk = 0;
+            if ((a.flag[n] & TYPE_MASK) == T_FLUID) {
+                const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
+                          z = (int)(n / L.nxy);
+                const Nbr nbh(L, x, y, z);
+                bool near = false;
+#pragma unroll
+                for (int j = 1; j < Q; ++j) near |= (a.flag[nbh.of(n, j)] & TYPE_MASK) == T_PARTICLE;
+                mk = near;
+            }
+            a.mark[c] = mk;
+        }
+        __syncthreads();
+        {
+            const int ch2 = (nc2 + SQ_THREADS - 1) / SQ_THREADS;
+            const int c0 = min(nc2, tid * ch2), c1 = min(nc2, c0 + ch2);
+            int cnt = 0;
+            for (int c = c0; c < c1; ++c) cnt += a.mark[c];
+            int off = 0;
+            Scan(scan_tmp).ExclusiveSum(cnt, off, sh_total);
+            __syncthreads();
+            for (int c = c0; c < c1; ++c) {
+                if (!a.mark[c]) continue;
+                const int n = a.cand[c];
+                if (off < a.link_cap) {
+                    a.links[off] = n;
+                    a.linkslot[n] = off;
+                    a.flag[n] |= NEAR_PARTICLE;
+                }
+                ++off;
+            }
+        }
+        __syncthreads();
+        if (tid == 0) {
+            s.n_links = min(sh_total, a.link_cap);
+            if (sh_total > a.link_cap) s.status |= ST_LINK_OVERFLOW;
+            a.shell_hdr->valid = 2;
+        }
+    }
+    __syncthreads();
+}
+
+// The state a run ends a step with, word by word. The wall force belongs to
+// k_finalize, and status bits are only ever added (the bulk's watchdog may set
+// one meanwhile).
+__device__ __forceinline__ void store_sq_state(SqState* dst, const SqState& s) {
+    constexpr int NS = (int)(sizeof(SqState) / 4);
+    constexpr int W0 = (int)(offsetof(SqState, wall_force) / 4), W1 = W0 + (int)(sizeof(SqState::wall_force) / 4);
+    constexpr int ST = (int)(offsetof(SqState, status) / 4);
+    const int t = threadIdx.x;
+    if (t < NS && !(t >= W0 && t < W1) && t != ST)
+        reinterpret_cast<uint32_t*>(dst)[t] = reinterpret_cast<const uint32_t*>(&s)[t];
+    if (t == ST && s.status) atomicOr(&dst->status, s.status);
+}
+
+// The rigid body (stage BODY), the sphere's box and what the remap's test needs
+// of the new centre. Warp 0 holds the components of X and U in its lanes 0-2,
+// warp 1 those of W and e, so that each division (most of the instructions
+// here) runs once for all components and the two chains side by side. The
+// values are the reference's, operation for operation.
+__device__ __forceinline__ void body_rotation(SqShared& sh) {   // warp 1
+    SqState& s = sh.s;
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, d = lane < 3 ? lane : 0, d1 = d == 2 ? 0 : d + 1, d2 = d == 0 ? 2 : d - 1;
+    // Squirmer::integrate (squirmer.cpp:52-68)
+    double w = s.W[d] + (s.Th[d] + s.Tc[d]) / s.I, e = s.e[d];
+    if (s.planar && d != 2) w = 0.0;
+    e += __shfl_sync(ALL, w, d1) * s.e[d2] - __shfl_sync(ALL, w, d2) * s.e[d1];
+    if (s.planar && d == 2) e = 0.0;
+    const double f0 = __shfl_sync(ALL, e, 0), f1 = __shfl_sync(ALL, e, 1), f2 = __shfl_sync(ALL, e, 2);
+    e /= sqrt(f0 * f0 + f1 * f1 + f2 * f2);
+    const bool bad = !(isfinite(w) && isfinite(e) && isfinite(s.Th[d]));
+    __syncwarp();   // every lane has read the old state
+    if (lane < 3) { s.W[d] = w; s.e[d] = e; s.Tc[d] = 0.0; }
+    if (__any_sync(ALL, bad) && lane == 0) atomicOr(&s.status, ST_NAN);
+}
+__device__ __forceinline__ void body_and_box(const Lattice& L, SqShared& sh, bool body, int shell_ok,
+                                             const double* shell_X) {   // warp 0
+    SqState& s = sh.s;
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, d = lane < 3 ? lane : 0;
+    const bool lin = lane < 3;
+    const int nd = d == 0 ? L.nx : (d == 1 ? L.ny : L.nz);
+    const bool walled = d == 1 ? L.walls_y != 0 : (d == 2 && L.walls_z != 0);
+    double X = s.X[d];
+    bool bad = false, far = false;
+    if (body) {
+        // LBM::applyWallPotential (lbm.cpp:231-241): the lower and the upper wall
+        double Fw = 0.0;
+        const double hl = X - s.R - 0.5, hu = (nd - 1.5) - X - s.R;
+        if (walled && hl < s.hc) Fw += soft_wall_force(hl, s.eps, s.FS, s.hc);
+        if (walled && hu < s.hc) Fw -= soft_wall_force(hu, s.eps, s.FS, s.hc);
+        // Squirmer::integrate (squirmer.cpp:52-68)
+        double v = s.U[d] + (s.Fh[d] + s.Fc[d] + Fw) / s.M;
+        if (s.planar && d == 2) v = 0.0;
+        const double Xold = X;
+        X += v;
+        // LBM::enforceMinimumGap (lbm.cpp:245-253)
+        bool hitl = false, hith = false;
+        if (lin && walled) {
+            const double lo = 0.5 + s.R + s.hmin, hi = (nd - 1.5) - s.R - s.hmin;
+            if (X < lo) { X = lo; if (v < 0) v = 0; hitl = true; }
+            if (X > hi) { X = hi; if (v > 0) v = 0; hith = true; }
+        }
+        bad = __any_sync(ALL, !(isfinite(X) && isfinite(v) && isfinite(s.Fh[d])));
+        // The densities the refill reads were stored for the box of the
+        // previous position widened by 2; that covers this step's box
+        // widened by 1 only if the centre moved less than one cell.
+        far = __any_sync(ALL, fabs(X - Xold) >= 1.0) && !bad;
+        const int hits = __popc(__ballot_sync(ALL, hitl)) + __popc(__ballot_sync(ALL, hith));
+        if (lin) { s.X[d] = X; s.U[d] = v; s.Fw[d] = Fw; s.Fc[d] = 0.0; }
+        if (lane == 0) {
+            s.t += 1;
+            s.contacts += hits;
+            if (bad || far) atomicOr(&s.status, bad ? ST_NAN : ST_REMAP_RANGE);
+        }
+    }
+    if (lin && !bad && !far) {
+        // the sphere's bounding box (lbm.cpp:272-276)
+        int b0 = (int)floor(X - s.R) - 2, b1 = (int)ceil(X + s.R) + 2;
+        if (d == 1 && walled) { b0 = max(0, b0); b1 = min(nd - 1, b1); }
+        sh.box[d] = b0;
+        sh.box[3 + d] = b1 - b0 + 1;
+        // the centre as a node index and a fraction of a cell, for the FP32 test
+        const double c0 = floor(X);
+        sh.cf[d] = (float)(X - c0);
+        double ci = c0;
+        if (!walled && !(c0 >= 0.0 && c0 < nd)) ci -= nd * floor(c0 / nd);
+        sh.ci[d] = (int)ci;
+        sh.wbox[d] = b0 >= 0 && b0 < nd ? b0 : ((b0 % nd) + nd) % nd;
+    }
+    const double q = X - shell_X[d];
+    const double q0 = __shfl_sync(ALL, q, 0), q1 = __shfl_sync(ALL, q, 1), q2 = __shfl_sync(ALL, q, 2);
+    if (lane == 0) sh.rebuild = !(shell_ok && q0 * q0 + q1 * q1 + q2 * q2 < SHELL_SLACK * SHELL_SLACK);
+}
+
+template <class S, bool PDL>
+__device__ __forceinline__ void squirmer_update(const Lattice& L, const SqArgs& a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ SqShared sh;
+    SqState& s = sh.s;
+    const int tid = threadIdx.x;
+    const bool early = PDL && (a.stages & STAGE_PRE) != 0;   // uniform
+    if (PDL && !early) pdl_wait();
+    {   // the state, one word per thread
+        constexpr int NS = (int)(sizeof(SqState) / 4);
+        static_assert(sizeof(SqState) % 4 == 0 && NS <= SQ_THREADS, "one word per thread");
+        if (tid < NS) reinterpret_cast<uint32_t*>(&s)[tid] = __ldcg(reinterpret_cast<const uint32_t*>(a.sq) + tid);
+    }
+    // the first candidates of the remap (see stage REMAP), their types and
+    // coordinates, kept in shared memory until the new centre is known
+    const bool remap = (a.stages & STAGE_REMAP) != 0;
+    int ncand = 0, shell_ok = 0;
+    double shell_X[3] = {0, 0, 0};
+    CandSh& cs = *reinterpret_cast<CandSh*>(smem_raw + FEW_BYTES);
+    if (remap) {
+        shell_ok = __ldcg(&a.shell_hdr->valid);
+        ncand = shell_ok ? __ldcg(&a.shell_hdr->n) : 0;
+        for (int d = 0; d < 3; ++d) shell_X[d] = __ldcg(&a.shell_hdr->X[d]);
+#pragma unroll 2
+        for (int c = tid; c < min(ncand, SQ_PRE * SQ_THREADS); c += SQ_THREADS) {
+            const unsigned n = (unsigned)__ldcg(a.shell + c);
+            cs.ty[c] = __ldcg(a.flag + n) & TYPE_MASK;
+            const unsigned q = n / (unsigned)L.nx, z = q / (unsigned)L.ny;
+            cs.n[c] = n;
+            cs.x[c] = (int)(n - q * (unsigned)L.nx);
+            cs.yz[c] = (q - z * (unsigned)L.ny) | z << 16;
+        }
+    }
+    if (tid == 0) {
+        sh.mass_delta = 0.0;
+        sh.dfluid = 0;
+        sh.few = 0;
+        sh.ncand = ncand;
+    }
+    if (early) pdl_wait();
+    if (PDL) pdl_launch_dependents();
+    __syncthreads();
+    if (s.status & (ST_NAN | ST_REMAP_RANGE | ST_LINK_OVERFLOW)) return;  // invalid already; the host reports it
+
+    const bool loop = (a.stages & STAGE_LOOP) != 0;
+    const bool corr_step = loop && a.corr_step;
+
+    // ---------------- stages FORCE, BODY ----------------
+    if (a.stages & STAGE_FORCE) block_sum_rows<6>(a.link_part, s.n_links, LINK_PART, 0, sh.sums);
+    const bool body = (a.stages & STAGE_BODY) != 0;
+    if (tid < 32) {
+        if ((a.stages & STAGE_FORCE) && tid < 3) s.Fh[tid] = sh.sums[tid];
+        __syncwarp();
+        body_and_box(L, sh, body, shell_ok, shell_X);
+    } else if (tid < 64) {
+        if ((a.stages & STAGE_FORCE) && tid < 35) s.Th[tid - 32] = sh.sums[tid - 29];
+        __syncwarp();
+        if (body) body_rotation(sh);
+    }
+    __syncthreads();
+    if (s.status & (ST_NAN | ST_REMAP_RANGE)) {
+        store_sq_state(a.sq, s);
+        return;
+    }
+
+    // ---------------- stage REMAP ----------------
+    // Candidates within the cached shell: each is first tested in FP32 (the
+    // squared distance is off by less than 1e-6 R^2 there); one within 1e-5 R^2
+    // + 1e-3 of the surface, or about half a lattice away, by the reference's
+    // FP64 offset. If few nodes change, remap_few does the rest.
+    if (remap) {
+        FewSh& w = *reinterpret_cast<FewSh*>(smem_raw);
+        bool walk = sh.rebuild != 0;   // uniform
+        if (!walk) {
+            const double R2 = s.R * s.R;
+            const float R2f = (float)R2, band = 1e-5f * R2f + 1e-3f;
+            const int hx = L.nx - 4, hy = L.walls_y ? 1 << 30 : L.ny - 4, hz = L.walls_z ? 1 << 30 : L.nz - 4;
+#pragma unroll 1
+            for (int c = tid; c < ncand; c += SQ_THREADS) {
+                unsigned n, ty;
+                int x, y, z;
+                if (c < SQ_PRE * SQ_THREADS) {
+                    n = cs.n[c]; ty = cs.ty[c];
+                    x = cs.x[c]; y = (int)(cs.yz[c] & 0xffffu); z = (int)(cs.yz[c] >> 16);
+                } else {
+                    n = (unsigned)a.shell[c]; ty = a.flag[n] & TYPE_MASK;
+                    x = (int)(n % (unsigned)L.nx); y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny); z = (int)(n / L.nxy);
+                }
+                if (ty == T_WALL) continue;
+                int dx = x - sh.ci[0], dy = y - sh.ci[1], dz = z - sh.ci[2];
+                if (2 * dx > L.nx) dx -= L.nx; else if (2 * dx < -L.nx) dx += L.nx;
+                if (!L.walls_y) { if (2 * dy > L.ny) dy -= L.ny; else if (2 * dy < -L.ny) dy += L.ny; }
+                if (!L.walls_z) { if (2 * dz > L.nz) dz -= L.nz; else if (2 * dz < -L.nz) dz += L.nz; }
+                const float ex = (float)dx - sh.cf[0], ey = (float)dy - sh.cf[1], ez = (float)dz - sh.cf[2];
+                const float gap = ex * ex + ey * ey + ez * ez - R2f;
+                bool inside = gap < 0.f;
+                if (fabsf(gap) < band || 2 * abs(dx) > hx || 2 * abs(dy) > hy || 2 * abs(dz) > hz) {
+                    double r[3];
+                    offset_from_squirmer(L, &s, x, y, z, r);
+                    inside = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] < R2;
+                }
+                if (inside != (ty == T_PARTICLE)) {
+                    const int k = atomicAdd(&sh.few, 1);
+                    if (k < SQ_FEW) {
+                        const int kx = x - sh.wbox[0], ky = y - sh.wbox[1], kz = z - sh.wbox[2];
+                        w.fnode[k] = n; w.fx[k] = x; w.fy[k] = y; w.fz[k] = z;
+                        w.fkind[k] = inside ? 1 : 2;
+                        // visit index in the box (z, y, x of the first visit)
+                        w.fkey[k] = ((kz < 0 ? kz + L.nz : kz) * sh.box[4] + (ky < 0 ? ky + L.ny : ky)) * sh.box[3] +
+                                    (kx < 0 ? kx + L.nx : kx);
+                    }
+                }
+            }
+        }
+        // meanwhile: the zones of the coming steps, from this box (see ZoneBox)
+        if (tid >= SQ_THREADS - 3) {
+            const int d = SQ_THREADS - 1 - tid, nd = d == 0 ? L.nx : (d == 1 ? L.ny : L.nz);
+            const bool wall_axis = d == 1 ? L.walls_y != 0 : (d == 2 && L.walls_z != 0);
+            const int wd = zone_width(s.R, nd, wall_axis);
+            int lo;
+            zone_axis(sh.box[d], nd, wd, wall_axis, lo);
+            if (a.zslot_a >= 0) { s.zone[a.zslot_a].w[d] = wd; s.zone[a.zslot_a].lo[d] = lo; }
+            if (a.zslot_b >= 0) { s.zone[a.zslot_b].w[d] = wd; s.zone[a.zslot_b].lo[d] = lo; }
+        }
+        __syncthreads();
+        const int nfew = sh.few;
+        walk = walk || (nfew > 0 && (nfew > SQ_FEW || shell_ok != 2 || s.n_links < 0 || s.n_links > SQ_FEW_LINKS));
+        if (walk) remap_walk<S>(L, a, sh, smem_raw, shell_ok, corr_step);   // uniform
+        else if (nfew > 0) remap_few<S>(L, a, sh, w, nfew, corr_step);
+        if (tid == 0) s.n_fluid += sh.dfluid;
     }
 
     // ---------------- stage LOOP ----------------
     double mstep = 0.0;
     if (corr_step) {
-        block_sum_rows<1>(a.block_part, a.nblocks, BLOCK_PART, 3, sums);
-        mstep = sums[0];
-        block_sum_rows<1>(a.block_part_b, a.nblocks_b, BLOCK_PART, 3, sums);
-        mstep += sums[0];
+        __syncthreads();
+        block_sum_rows<1>(a.block_part, a.nblocks, BLOCK_PART, 3, sh.sums);
+        mstep = sh.sums[0];
+        __syncthreads();
+        block_sum_rows<1>(a.block_part_b, a.nblocks_b, BLOCK_PART, 3, sh.sums);
+        mstep += sh.sums[0];
         if (a.nblocks_w > 0) {
-            block_sum_rows<1>(a.block_part_w, a.nblocks_w, BLOCK_PART, 3, sums);
-            mstep += sums[0];
+            __syncthreads();
+            block_sum_rows<1>(a.block_part_w, a.nblocks_w, BLOCK_PART, 3, sh.sums);
+            mstep += sh.sums[0];
         }
     }
     if (tid == 0) {
+        s.corr_pending = 0;
         if (loop) {
-            s.corr_pending = 0;
             if (corr_step && s.n_fluid > 0) {
                 // LBM::correctMass (lbm.cpp:324-339): d = 1 - m / n_fluid, with m
                 // the populations summed after this step and its remap.
-                const double m = mstep + sh_mass_delta;
+                const double m = mstep + sh.mass_delta;
                 s.corr_d = S::shifted ? -(m / (double)s.n_fluid) : 1.0 - m / (double)s.n_fluid;
                 s.corr_pending = 1;
             }
-            if (s.traj_every > 0 && s.t % s.traj_every == 0) {
-                double* row = a.traj + (size_t)(s.traj_count % TRAJ_RING) * TRAJ_COLS;
-                row[0] = (double)s.t;
+            const bool row = s.traj_every > 0 && ((unsigned long long)s.t <= 0xffffffffull
+                                                      ? (unsigned)s.t % (unsigned)s.traj_every == 0
+                                                      : s.t % s.traj_every == 0);
+            if (row) {
+                double* out = a.traj + (size_t)(s.traj_count % TRAJ_RING) * TRAJ_COLS;
+                out[0] = (double)s.t;
                 for (int d = 0; d < 3; ++d) {
-                    row[1 + d] = s.X[d]; row[4 + d] = s.e[d]; row[7 + d] = s.U[d]; row[10 + d] = s.W[d];
+                    out[1 + d] = s.X[d]; out[4 + d] = s.e[d]; out[7 + d] = s.U[d]; out[10 + d] = s.W[d];
                 }
-                row[13] = s.Fw[1]; row[14] = s.Fw[2];
+                out[13] = s.Fw[1]; out[14] = s.Fw[2];
                 s.traj_count += 1;
             }
-        } else {
-            s.corr_pending = 0;
         }
-        // zones of the coming steps, from this box (see ZoneBox)
-        const int blo[3] = {bx0, by0, bz0};
-        const int nd[3] = {L.nx, L.ny, L.nz};
-        const bool wall_axis[3] = {false, L.walls_y != 0, L.walls_z != 0};
-        for (int slot : {a.zslot_a, a.zslot_b}) {
-            if (slot < 0) continue;
-            for (int d = 0; d < 3; ++d) {
-                s.zone[slot].w[d] = zone_width(s.R, nd[d], wall_axis[d]);
-                zone_axis(blo[d], nd[d], s.zone[slot].w[d], wall_axis[d], s.zone[slot].lo[d]);
-            }
-        }
-        *a.sq = s;
     }
+    __syncthreads();
+    store_sq_state(a.sq, s);
 }
 
 template <class S>
-__global__ void __launch_bounds__(SQ_THREADS) k_squirmer(const Lattice L, const SqArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
-    squirmer_update<S>(L, a);
+__global__ void __launch_bounds__(SQ_THREADS) k_squirmer(const __grid_constant__ Lattice L,
+                                                         const __grid_constant__ SqArgs a) {
+    squirmer_update<S, true>(L, a);
 }
 
 // Ensemble: one CTA per member, each with its own lattice and arguments; the
@@ -696,7 +1117,7 @@ __global__ void __launch_bounds__(SQ_THREADS) k_squirmer_batch(const Lattice* la
         }
     }
     __syncthreads();
-    squirmer_update<S>(L, A);
+    squirmer_update<S, false>(L, A);
 }
 
 }  // namespace lbmgpu

@@ -62,13 +62,24 @@ namespace lbmgpu {
 constexpr int BOUNDARY_BLOCK = 64;
 constexpr int ZONE_MAX_REGS = 128;
 
+// r - n round(r / n), bit for bit, without the FP64 division in the usual case:
+// the multiple k of n is guessed in FP32, and where r - n k lies within 0.499 n
+// of zero (r - n k is exact to a rounding, k n being a small integer) r / n is
+// closer to k than to any half-integer, so round(r / n) is k. Otherwise (a node
+// about half a lattice away) the division decides.
+__device__ __forceinline__ double min_image(double r, int n) {
+    const double t = r - n * (double)rintf(__fdividef((float)r, (float)n));
+    if (fabs(t) < 0.499 * n) return t;
+    return r - n * round(r / n);
+}
+
 // LBM::offsetFromSquirmer (lbm.cpp:100-104): minimum image in x always, in
 // y/z only where there is no wall.
 __device__ __forceinline__ void offset_from_squirmer(const Lattice& L, const SqState* s, double px,
                                                      double py, double pz, double r[3]) {
-    r[0] = px - s->X[0]; r[0] -= L.nx * round(r[0] / L.nx);
-    r[1] = py - s->X[1]; if (!L.walls_y) r[1] -= L.ny * round(r[1] / L.ny);
-    r[2] = pz - s->X[2]; if (!L.walls_z) r[2] -= L.nz * round(r[2] / L.nz);
+    r[0] = min_image(px - s->X[0], L.nx);
+    r[1] = py - s->X[1]; if (!L.walls_y) r[1] = min_image(r[1], L.ny);
+    r[2] = pz - s->X[2]; if (!L.walls_z) r[2] = min_image(r[2], L.nz);
 }
 
 // Squirmer::surfaceVelocity (squirmer.cpp:35-46): U + W x r, plus the Blake

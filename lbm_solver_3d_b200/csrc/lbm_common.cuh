@@ -209,7 +209,8 @@ struct SqState {
 struct ShellCache {
     double X[3];   // reference centre (unwrapped, like SqState::X)
     int n;         // candidates in the list
-    int valid;     // 0: rebuild on the next remap
+    int valid;     // 0: rebuild on the next remap; 1: the list holds; 2: and the link list
+                   // was rebuilt by the update itself (a loaded one is not edited until then)
 };
 constexpr double SHELL_SLACK = 0.75;
 

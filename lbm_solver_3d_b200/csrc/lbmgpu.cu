@@ -526,7 +526,7 @@ void issue_fused(lbmgpu_handle* h, cudaStream_t sa, cudaStream_t sb, const StepP
     if (h->has_sq) {
         if (sp.corr) cudaStreamWaitEvent(sb, h->ev_b[sp.s & 1], 0);
         const int za = (int)((sp.s + 2) % ZONE_SLOTS);
-        h->lz->squirmer(h->L, squirmer_args(h, par ^ 1, STAGE_FORCE | STAGE_BODY | STAGE_REMAP | STAGE_LOOP,
+        h->lz->squirmer(h->L, squirmer_args(h, par ^ 1, STAGE_PRE | STAGE_FORCE | STAGE_BODY | STAGE_REMAP | STAGE_LOOP,
                                             sp.corr ? 1 : 0, za, -1), sb);
         cudaEventRecord(h->ev_s, sb);
         ++k;
