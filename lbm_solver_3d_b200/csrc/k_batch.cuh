@@ -1291,11 +1291,13 @@ __global__ void __launch_bounds__(BOUNDARY_BLOCK) k_zone_batch(const Lattice* __
     }
     __syncthreads();
     __shared__ __align__(16) SqState zsq;
-    __shared__ LinkStash<S> stash[Q * BOUNDARY_BLOCK];
+    __shared__ ZoneWarp<S> zw[BOUNDARY_BLOCK / 32];
     copy_sq_state(&zsq, A.sq);
     __syncthreads();
+    const ZoneBox& zb = zsq.zone[st.zslot];
     NodeSums sums;
-    zone_cell<S, PAR, true, MACRO>(L, A, blk * BOUNDARY_BLOCK + threadIdx.x, sums, &zsq, stash);
+    zone_cell<S, PAR, true, MACRO>(L, A, blk * BOUNDARY_BLOCK + threadIdx.x, zb.lo[0], zb.lo[1], zb.lo[2], sums, &zsq,
+                                   &zw[threadIdx.x >> 5], [] {});
     if (MACRO || st.do_mass)
         block_reduce4<BOUNDARY_BLOCK>(sums.fw[0], sums.fw[1], sums.fw[2], sums.mass,
                                       zone_part + ((size_t)m * gzmax + blk) * BLOCK_PART);

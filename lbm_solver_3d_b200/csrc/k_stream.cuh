@@ -171,10 +171,19 @@ struct NodeSums {
     double rho = 0;       // GENERAL: the node's density, for zone_particle_links
 };
 
-// Post-collision values of a zone block's particle links, [direction][thread]:
+// Post-collision values of a zone warp's particle links, [direction][lane]:
 // the population itself (FP64) or its deviation (shifted forms).
 template <class S>
 using LinkStash = typename S::A;
+
+// A zone warp's shared memory: the values above, the list of its particle
+// links (lane | direction << 8, ascending), and one round's results.
+template <class S>
+struct ZoneWarp {
+    double res[32][7];
+    LinkStash<S> stash[Q * 32];
+    uint16_t item[32 * (Q - 1)];
+};
 
 // ---------------------------------------------------------------------------
 //  update_node: the whole LBM::step body for one fluid node n.
@@ -438,8 +447,8 @@ __device__ __forceinline__ void plain_pairs(const Lattice& L, typename S::T* __r
 }
 
 // GENERAL: the particle links are not computed here. Their post-collision
-// values go to link_stash[i * BOUNDARY_BLOCK + threadIdx.x], their directions
-// to out.pmask, and zone_particle_links finishes them with the whole warp.
+// values go to link_stash[i * 32 + lane], their directions to out.pmask, and
+// zone_particle_links finishes them with the whole warp.
 // FP64 collide and push of a node with only fluid neighbours, in the
 // reference's arithmetic (lbm.cpp:162-172, every operation in its order, no
 // contraction), one opposite pair (i, i+1) at a time. The terms of i+1 are
@@ -604,7 +613,7 @@ __device__ __forceinline__ void update_node(const Lattice& L, const StreamArgs& 
                 continue;
             }
             if (GENERAL && tt == T_PARTICLE) {   // finished by zone_particle_links
-                link_stash[i * BOUNDARY_BLOCK + threadIdx.x] = fpost;
+                link_stash[i * 32 + (threadIdx.x & 31)] = fpost;
                 out.pmask |= 1u << i;
                 continue;
             }
@@ -665,7 +674,7 @@ __device__ __forceinline__ void update_node(const Lattice& L, const StreamArgs& 
                     continue;
                 }
                 if (GENERAL && tt == T_PARTICLE) {   // finished by zone_particle_links
-                    link_stash[i * BOUNDARY_BLOCK + threadIdx.x] = dpost;
+                    link_stash[i * 32 + (threadIdx.x & 31)] = dpost;
                     out.pmask |= 1u << i;
                     continue;
                 }
@@ -990,86 +999,139 @@ __global__ void __launch_bounds__(PAIR_BLOCK, 4) k_bulk_pair(const Lattice L, co
 // ---------------------------------------------------------------------------
 // The particle links left by update_node<GENERAL> (lbm.cpp:189-215 with u_b
 // = U + W x r_b + slip, r_b at the link midpoint), finished by the whole warp
-// (every lane calls it): in round k each lane takes its k-th link in
-// ascending direction order, so the warp runs as many rounds as its busiest
-// lane has links instead of one pass per direction that any lane needs. The
-// arithmetic and the order of the per-node sums are those of the direction
-// loop in update_node.
+// (every lane calls it): the warp's links, lane by lane in ascending direction
+// order, are numbered and dealt out 32 at a time, so a round costs one link's
+// latency (a square root, three divisions) whichever lanes the links belong to;
+// a node with 9 links cost its warp 9 rounds. Each lane then adds its own
+// links' results in direction order: the arithmetic and the order of the
+// per-node sums are those of the direction loop in update_node.
+// Zone kernel alone, with this and the populations loaded beside the types:
+// 11.2 -> 8.3 us (64x34x32, R = 4, FP64), 13.5 -> 9.0 us (256x128x128, R = 8,
+// FP32); the kernel is bound by its latencies (launch, four rounds of
+// dependent loads, the FP64 chains), not by bytes.
 template <class S, int PAR>
 __device__ __forceinline__ void zone_particle_links(const Lattice& L, const StreamArgs& a, const SqState* sq,
-                                                    unsigned n, int x, int y, int z, bool do_mass,
-                                                    const LinkStash<S>* stash, NodeSums& out) {
+                                                    unsigned n, int x, int y, int z, bool do_mass, ZoneWarp<S>* w,
+                                                    NodeSums& out) {
     using T = typename S::T;
     T* __restrict__ f = static_cast<T*>(a.f);
-    unsigned m = out.pmask;
-    const int rounds = __reduce_max_sync(0xffffffffu, (unsigned)__popc(m));
-    for (int k = 0; k < rounds; ++k) {
-        if (!m) continue;
-        const int i = __ffs(m) - 1;
-        m &= m - 1;
-        const int cx = c_cx[i], cy = c_cy[i], cz = c_cz[i];
-        const double w = c_w[i];
-        T* local = f + (size_t)opp_rt(i) * L.N + n;
-        T* remote = f + (size_t)i * L.N + nbr_rt(L, x, y, z, cx, cy, cz);
-        double rb[3], ub[3];
-        offset_from_squirmer(L, sq, x + 0.5 * cx, y + 0.5 * cy, z + 0.5 * cz, rb);
-        surface_velocity(sq, rb, ub, true);
-        const double cub = cx * ub[0] + cy * ub[1] + cz * ub[2];
-        double sm, dl;
-        if constexpr (!S::shifted) {
-            const double fpost = stash[i * BOUNDARY_BLOCK + threadIdx.x];
-            const double fb = fpost - 6.0 * w * out.rho * cub;
-            S::st(PAR == 0 ? remote : local, fb);
-            if (do_mass) out.mass += fb;
-            sm = fpost + fb;
-            dl = fpost - fb;
-        } else {
-            const float dpost = stash[i * BOUNDARY_BLOCK + threadIdx.x];   // storage units
-            dl = 6.0 * w * out.rho * cub;   // fpost - fb (deviation units)
-            const float dfb = (float)((double)dpost - dl * S::SC);
-            S::st(PAR == 0 ? remote : local, dfb);
-            if (do_mass) out.mass += (double)S::rt(dfb) * S::INV;
-            const double fpost = w + (double)dpost * S::INV;
-            sm = 2.0 * fpost - dl;            // fpost + fb
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, cnt = __popc(out.pmask);
+    if (!__any_sync(ALL, cnt)) return;
+    int end = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(ALL, end, o);
+        if (lane >= o) end += v;
+    }
+    const int begin = end - cnt, total = __shfl_sync(ALL, end, 31);
+    {
+        int k = begin;
+#pragma unroll 1
+        for (unsigned m = out.pmask; m; m &= m - 1) w->item[k++] = (uint16_t)(lane | (__ffs(m) - 1) << 8);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int base = 0; base < total; base += 32) {
+        const bool on = base + lane < total;
+        const int it = on ? w->item[base + lane] : 0;
+        const int src = it & 31, i = it >> 8;
+        const int xs = __shfl_sync(ALL, x, src), ys = __shfl_sync(ALL, y, src), zs = __shfl_sync(ALL, z, src);
+        const unsigned ns = __shfl_sync(ALL, n, src);
+        const double rho = __shfl_sync(ALL, out.rho, src);
+        if (on) {
+            const int cx = c_cx[i], cy = c_cy[i], cz = c_cz[i];
+            const double wi = c_w[i];
+            T* local = f + (size_t)opp_rt(i) * L.N + ns;
+            T* remote = f + (size_t)i * L.N + nbr_rt(L, xs, ys, zs, cx, cy, cz);
+            double rb[3], ub[3];
+            offset_from_squirmer(L, sq, xs + 0.5 * cx, ys + 0.5 * cy, zs + 0.5 * cz, rb);
+            surface_velocity(sq, rb, ub, true);
+            const double cub = cx * ub[0] + cy * ub[1] + cz * ub[2];
+            double sm, dl, mass;
+            if constexpr (!S::shifted) {
+                const double fpost = w->stash[i * 32 + src];
+                const double fb = fpost - 6.0 * wi * rho * cub;
+                S::st(PAR == 0 ? remote : local, fb);
+                mass = fb;
+                sm = fpost + fb;
+                dl = fpost - fb;
+            } else {
+                const float dpost = w->stash[i * 32 + src];   // storage units
+                dl = 6.0 * wi * rho * cub;   // fpost - fb (deviation units)
+                const float dfb = (float)((double)dpost - dl * S::SC);
+                S::st(PAR == 0 ? remote : local, dfb);
+                mass = (double)S::rt(dfb) * S::INV;
+                const double fpost = wi + (double)dpost * S::INV;
+                sm = 2.0 * fpost - dl;            // fpost + fb
+            }
+            const double dpx = sm * cx - dl * ub[0];
+            const double dpy = sm * cy - dl * ub[1];
+            const double dpz = sm * cz - dl * ub[2];
+            double* r = w->res[lane];
+            r[0] = dpx; r[1] = dpy; r[2] = dpz;
+            r[3] = rb[1] * dpz - rb[2] * dpy;
+            r[4] = rb[2] * dpx - rb[0] * dpz;
+            r[5] = rb[0] * dpy - rb[1] * dpx;
+            r[6] = mass;
         }
-        const double dpx = sm * cx - dl * ub[0];
-        const double dpy = sm * cy - dl * ub[1];
-        const double dpz = sm * cz - dl * ub[2];
-        out.fp[0] += dpx; out.fp[1] += dpy; out.fp[2] += dpz;
-        out.tp[0] += rb[1] * dpz - rb[2] * dpy;
-        out.tp[1] += rb[2] * dpx - rb[0] * dpz;
-        out.tp[2] += rb[0] * dpy - rb[1] * dpx;
+        __syncwarp();
+#pragma unroll 1
+        for (int k = max(begin, base); k < min(end, base + 32); ++k) {
+            const double* r = w->res[k - base];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) { out.fp[d] += r[d]; out.tp[d] += r[3 + d]; }
+            if (do_mass) out.mass += r[6];
+        }
+        __syncwarp();
     }
 }
 
-// Cell k of the zone, one per thread (every thread of the block calls it);
+// Populations already in registers (zone_cell loads them before it knows the
+// node's type).
+template <class V>
+struct HeldSrc {
+    const V* held;
+    template <class S, int PAR, class W>
+    __device__ __forceinline__ void load(const typename S::T*, unsigned, unsigned, const Nbr&, W* v) const {
+#pragma unroll
+        for (int i = 0; i < Q; ++i) v[i] = held[i];
+    }
+};
+
+// Cell k of the zone whose corner is (lx, ly, lz), one per thread (every lane
+// of the warp calls it; sync() runs before the particle links read sq);
 // returns the sums for the block reduction. sq is the block's copy of the
-// squirmer state, stash the block's particle-link values.
-template <class S, int PAR, bool SQ, bool MACRO>
-__device__ __forceinline__ void zone_cell(const Lattice& L, const StreamArgs& a, int k, NodeSums& sums,
-                                          const SqState* sq, LinkStash<S>* stash) {
+// squirmer state, w the warp's shared memory. The node's populations are
+// loaded together with its type, so one memory latency covers both; a cell
+// that is not fluid loads them for nothing.
+template <class S, int PAR, bool SQ, bool MACRO, class Sync>
+__device__ __forceinline__ void zone_cell(const Lattice& L, const StreamArgs& a, int k, int lx, int ly, int lz,
+                                          NodeSums& sums, const SqState* sq, ZoneWarp<S>* w, Sync&& sync) {
     bool active = false;
     unsigned n = 0;
     int x = 0, y = 0, z = 0;
+    uint8_t fl = T_WALL;
+    using V = std::conditional_t<S::shifted, float, double>;
+    V held[Q];
     if (SQ && k < a.zone_cells) {
-        const ZoneBox* zb = &sq->zone[a.zslot];
         const int bx = k % a.zw[0], by = (k / a.zw[0]) % a.zw[1], bz = k / (a.zw[0] * a.zw[1]);
-        x = zb->lo[0] + bx; if (x >= L.nx) x -= L.nx;
-        y = zb->lo[1] + by; z = zb->lo[2] + bz;
+        x = lx + bx; if (x >= L.nx) x -= L.nx;
+        y = ly + by; z = lz + bz;
         if (L.walls_y) active = y >= 0 && y < L.ny; else { if (y >= L.ny) y -= L.ny; active = true; }
         if (L.walls_z) active = active && z >= 0 && z < L.nz; else if (z >= L.nz) z -= L.nz;
         if (active) {
             n = (unsigned)x + (unsigned)L.nx * ((unsigned)y + (unsigned)L.ny * (unsigned)z);
-            active = (a.flag[n] & TYPE_MASK) == T_FLUID;
+            fl = a.flag[n];
+            load_node<S, PAR>(static_cast<const typename S::T*>(a.f), L.N, n, Nbr(L, x, y, z), held);
+            active = (fl & TYPE_MASK) == T_FLUID;
         }
     }
-    uint8_t fl = 0;
-    if (active) {
-        fl = a.flag[n];
-        update_node<S, PAR, true, MACRO>(L, a, n, x, y, z, fl, 0, SQ || MACRO, sums, GlobalSrc(), stash);
-    }
+    if (active)
+        update_node<S, PAR, true, MACRO>(L, a, n, x, y, z, fl, 0, SQ || MACRO, sums, HeldSrc<V>{held}, w->stash);
+    sync();
     if (SQ) {
-        zone_particle_links<S, PAR>(L, a, sq, n, x, y, z, a.do_mass != 0, stash, sums);
+        zone_particle_links<S, PAR>(L, a, sq, n, x, y, z, a.do_mass != 0, w, sums);
         if (active && (fl & NEAR_PARTICLE)) {
             double* lp = a.link_part + (size_t)a.linkslot[n] * LINK_PART;
             lp[0] = sums.fp[0]; lp[1] = sums.fp[1]; lp[2] = sums.fp[2];
@@ -1091,11 +1153,15 @@ __global__ void __maxnreg__(ZONE_MAX_REGS) k_zone(const Lattice L, const StreamA
     pdl_wait();
     pdl_launch_dependents();
     __shared__ __align__(16) SqState zsq;
-    __shared__ LinkStash<S> stash[Q * BOUNDARY_BLOCK];
-    if (SQ) copy_sq_state(&zsq, a.sq);
-    __syncthreads();
+    __shared__ ZoneWarp<S> zw[BOUNDARY_BLOCK / 32];
+    int lo[3] = {0, 0, 0};
+    if (SQ) {
+        for (int d = 0; d < 3; ++d) lo[d] = a.sq->zone[a.zslot].lo[d];
+        copy_sq_state(&zsq, a.sq);   // read by the particle links only
+    }
     NodeSums sums;
-    zone_cell<S, PAR, SQ, MACRO>(L, a, blockIdx.x * BOUNDARY_BLOCK + threadIdx.x, sums, &zsq, stash);
+    zone_cell<S, PAR, SQ, MACRO>(L, a, blockIdx.x * BOUNDARY_BLOCK + threadIdx.x, lo[0], lo[1], lo[2], sums, &zsq,
+                                 &zw[threadIdx.x >> 5], [] { __syncthreads(); });
     if (MACRO || a.do_mass)
         block_reduce4<BOUNDARY_BLOCK>(sums.fw[0], sums.fw[1], sums.fw[2], sums.mass,
                                       a.block_part_b + (size_t)blockIdx.x * BLOCK_PART);
