@@ -17,7 +17,7 @@ __global__ void k_fill_rest(const Lattice L, void* f) {
     const size_t total = (size_t)Q * L.N;
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
         const int i = (int)(k / L.N);
-        Pop<S>::put(f, k, i, c_w[i]);
+        Pop<S>::put(f, k, i, w_rt(i));
     }
 }
 
@@ -26,7 +26,7 @@ template <class S>
 __global__ void k_get_pop(const Lattice L, const void* f, const uint8_t* flag, const SqState* sq, int P, int i,
                           double* out) {
     const int pend = sq->corr_pending;
-    const double add = pend ? c_w[i] * sq->corr_d : 0.0;
+    const double add = pend ? w_rt(i) * sq->corr_d : 0.0;
     for (unsigned n = blockIdx.x * blockDim.x + threadIdx.x; n < L.N; n += gridDim.x * blockDim.x) {
         const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny), z = (int)(n / L.nxy);
         double v = Pop<S>::get(f, logical_slot(L, P, i, n, x, y, z), i);
@@ -97,7 +97,7 @@ __global__ void k_mass_apply(const Lattice L, void* f, const uint8_t* flag, int 
         const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny), z = (int)(n / L.nxy);
         for (int i = 0; i < Q; ++i) {
             const size_t k = logical_slot(L, P, i, n, x, y, z);
-            Pop<S>::put(f, k, i, Pop<S>::get(f, k, i) + c_w[i] * d);
+            Pop<S>::put(f, k, i, Pop<S>::get(f, k, i) + w_rt(i) * d);
         }
     }
 }

@@ -449,27 +449,6 @@ __device__ __forceinline__ void span16(const void* p, size_t bytes, uintptr_t& s
     len = (unsigned)((a + bytes - start + 15) & ~(uintptr_t)15);
 }
 
-// velocity set by a runtime index (lanes of the producer take one direction each)
-__device__ __forceinline__ int c_opp_rt(int i) { return i == 0 ? 0 : ((i & 1) ? i + 1 : i - 1); }
-__device__ __forceinline__ int c_cx_rt(int i) {
-    int v = 0;
-#pragma unroll
-    for (int k = 0; k < Q; ++k) if (k == i) v = CX(k);
-    return v;
-}
-__device__ __forceinline__ int c_cy_rt(int i) {
-    int v = 0;
-#pragma unroll
-    for (int k = 0; k < Q; ++k) if (k == i) v = CY(k);
-    return v;
-}
-__device__ __forceinline__ int c_cz_rt(int i) {
-    int v = 0;
-#pragma unroll
-    for (int k = 0; k < Q; ++k) if (k == i) v = CZ(k);
-    return v;
-}
-
 // populations of node x from a stage (see update_node's Src parameter)
 template <class T>
 struct StagedSrc {
@@ -568,9 +547,9 @@ __global__ void __launch_bounds__(STAGED_THREADS) k_bulk_staged(const Lattice* _
                 const int i = lane;
                 int ys = rr.y, zs = rr.z, arr = i;
                 if (PAR == 1) {
-                    arr = c_opp_rt(i);
-                    ys = rr.y - c_cy_rt(i); if (ys < 0) ys += L.ny; else if (ys >= L.ny) ys -= L.ny;
-                    zs = rr.z - c_cz_rt(i); if (zs < 0) zs += L.nz; else if (zs >= L.nz) zs -= L.nz;
+                    arr = opp_rt(i);
+                    ys = rr.y - cy_rt(i); if (ys < 0) ys += L.ny; else if (ys >= L.ny) ys -= L.ny;
+                    zs = rr.z - cz_rt(i); if (zs < 0) zs += L.nz; else if (zs >= L.nz) zs -= L.nz;
                 }
                 const T* f = static_cast<const T*>(recA[slot].f);
                 span16(f + (size_t)arr * L.N + (size_t)L.nx * (ys + (size_t)L.ny * zs), (size_t)L.nx * sizeof(T), start,
@@ -788,9 +767,9 @@ __global__ void __launch_bounds__(RUNS_THREADS, 2) k_bulk_runs(const Lattice* __
                 const int i = lane;
                 int ys = run.y, zs = run.z, arr = i;
                 if (PAR == 1) {
-                    arr = c_opp_rt(i);
-                    ys = run.y - c_cy_rt(i); if (ys < 0) ys += L.ny; else if (ys >= L.ny) ys -= L.ny;
-                    zs = run.z - c_cz_rt(i); if (zs < 0) zs += L.nz; else if (zs >= L.nz) zs -= L.nz;
+                    arr = opp_rt(i);
+                    ys = run.y - cy_rt(i); if (ys < 0) ys += L.ny; else if (ys >= L.ny) ys -= L.ny;
+                    zs = run.z - cz_rt(i); if (zs < 0) zs += L.nz; else if (zs >= L.nz) zs -= L.nz;
                 }
                 const T* f = static_cast<const T*>(recA[slot].f);
                 span16(f + (size_t)arr * L.N + (size_t)L.nx * (ys + (size_t)L.ny * zs), cnt * sizeof(T), start, len, ob);
@@ -954,9 +933,9 @@ __device__ __forceinline__ void stage_row(const Lattice& L, const StreamArgs& a,
         const int i = lane;
         int ys = y, zs = z, arr = i;
         if (PAR == 1) {
-            arr = c_opp_rt(i);
-            ys = y - c_cy_rt(i); if (ys < 0) ys += L.ny; else if (ys >= L.ny) ys -= L.ny;
-            zs = z - c_cz_rt(i); if (zs < 0) zs += L.nz; else if (zs >= L.nz) zs -= L.nz;
+            arr = opp_rt(i);
+            ys = y - cy_rt(i); if (ys < 0) ys += L.ny; else if (ys >= L.ny) ys -= L.ny;
+            zs = z - cz_rt(i); if (zs < 0) zs += L.nz; else if (zs >= L.nz) zs -= L.nz;
         }
         const T* f = static_cast<const T*>(a.f);
         bulk_g2s_hint(sb + (size_t)i * nx * sizeof(T), f + (size_t)arr * L.N + (size_t)nx * (ys + (size_t)L.ny * zs),
@@ -1249,8 +1228,8 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX / 2, Rows2Cfg<S>::MINB) k_bul
                     const int i = lane;
                     int yd = y, zd = z;
                     if (PAR == 1) {
-                        yd = y + c_cy_rt(i); if (yd < 0) yd += L.ny; else if (yd >= L.ny) yd -= L.ny;
-                        zd = z + c_cz_rt(i); if (zd < 0) zd += L.nz; else if (zd >= L.nz) zd -= L.nz;
+                        yd = y + cy_rt(i); if (yd < 0) yd += L.ny; else if (yd >= L.ny) yd -= L.ny;
+                        zd = z + cz_rt(i); if (zd < 0) zd += L.nz; else if (zd >= L.nz) zd -= L.nz;
                     }
                     bulk_s2g_hint(fw + (size_t)i * L.N + (size_t)nx * (yd + (size_t)L.ny * zd), sb + (size_t)i * nx,
                                   (unsigned)(nx * sizeof(T)), l2_evict_first());

@@ -42,7 +42,7 @@ constexpr int SQ_THREADS = 512;
 constexpr int SQ_BATCH = 256;
 constexpr int SQ_SORT_CAP = 2048;   // changes ordered in shared memory (3 ints each)
 constexpr int SQ_GROUP = 4;         // remap candidates tested per thread with their loads in flight together
-constexpr int SQ_PRE = 6;           // candidates per thread fetched ahead: 3072 of them, the shell up to R = 8
+constexpr int SQ_PRE = 8;           // candidates per thread fetched ahead: 4096 of them, the shell up to R = 9
 constexpr int SQ_FEW = 32;          // changed nodes that remap_few orders: one warp
 constexpr int SQ_FEW_LINKS = 4096;  // boundary links that remap_few edits in shared memory (R up to about 12)
 constexpr int STAGE_BODY = 1, STAGE_REMAP = 2, STAGE_LOOP = 4, STAGE_FORCE = 8;
@@ -99,50 +99,70 @@ __device__ __forceinline__ double soft_wall_force(double h, double eps, double F
     return eps * FS * s * s;
 }
 
-// Deterministic block sum of NC (<= 8) columns over rows of a strided array:
-// each thread its rows in order, a shuffle tree per warp, the warps in order.
-// Short loops: the code runs once per step, from a cold instruction cache.
-template <int NC>
-__device__ __forceinline__ void block_sum_rows(const double* base, int rows, int stride, int col0, double* out_sh) {
-    __shared__ double red[SQ_THREADS / 32][8];
-    double acc[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) acc[c] = 0.0;
-    constexpr int U = NC > 1 ? 1 : 8;   // rows per thread with their loads in flight together
+// Deterministic block sum of one column of a strided array: each thread its
+// rows in order, a shuffle tree per warp, the warps in order.
+__device__ __forceinline__ void block_sum_rows(const double* base, int rows, int stride, int col, double* out_sh) {
+    __shared__ double red[SQ_THREADS / 32];
+    double acc = 0.0;
+    constexpr int U = 8;   // rows per thread with their loads in flight together
 #pragma unroll 1
     for (int k0 = threadIdx.x; k0 < rows; k0 += U * SQ_THREADS) {
-        double v[U][NC];
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + u * SQ_THREADS;
+            v[u] = k < rows ? base[(size_t)k * stride + col] : 0.0;
+        }
 #pragma unroll
         for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const int k = k0 + u * SQ_THREADS;
-                v[u][c] = k < rows ? base[(size_t)k * stride + col0 + c] : 0.0;
-            }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (k0 + u * SQ_THREADS < rows)
-#pragma unroll
-                for (int c = 0; c < NC; ++c) acc[c] += v[u][c];
+            if (k0 + u * SQ_THREADS < rows) acc += v[u];
     }
-#pragma unroll 1
-    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int c = 0; c < NC; ++c) acc[c] += __shfl_down_sync(0xffffffffu, acc[c], o);
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < SQ_THREADS / 32; ++w) t += red[w];
+        *out_sh = t;
+    }
+    __syncthreads();
+}
+
+// The link rows' sums (six columns of `cap` rows each), up to the warps: red[w]
+// gets warp w's. In the first level of the tree the half-warps exchange three
+// columns each, so that every later level moves three columns instead of six
+// (the shuffles are what this stage waits for).
+__device__ __forceinline__ void link_warp_sums(const double* part, int rows, size_t cap, double (*red)[6]) {
+    constexpr unsigned ALL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0)
+    double acc[6] = {0, 0, 0, 0, 0, 0}, half[3] = {0, 0, 0};
+    if (wid * 32 < rows) {   // a warp without rows adds 0
+#pragma unroll 2
+        for (int k = threadIdx.x; k < rows; k += SQ_THREADS)
 #pragma unroll
-        for (int c = 0; c < NC; ++c) red[wid][c] = acc[c];
-    __syncthreads();
-    if (threadIdx.x < NC) {   // one thread per column, the warps in order
-        double v[SQ_THREADS / 32], s = 0.0;
+            for (int c = 0; c < 6; ++c) acc[c] += part[c * cap + k];
+        const bool hi = lane >= 16;
 #pragma unroll
-        for (int w = 0; w < SQ_THREADS / 32; ++w) v[w] = red[w][threadIdx.x];
+        for (int c = 0; c < 3; ++c)
+            half[c] = (hi ? acc[3 + c] : acc[c]) + __shfl_xor_sync(ALL, hi ? acc[c] : acc[3 + c], 16);
 #pragma unroll
-        for (int w = 0; w < SQ_THREADS / 32; ++w) s += v[w];
-        out_sh[threadIdx.x] = s;
+        for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) half[c] += __shfl_down_sync(ALL, half[c], o, 16);
     }
-    __syncthreads();
+    if ((lane & 15) == 0)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) red[wid][(lane >> 4) * 3 + c] = half[c];
+}
+__device__ __forceinline__ double link_total(const double (*red)[6], int c) {   // the warps in order
+    double v[SQ_THREADS / 32], t = 0.0;
+#pragma unroll
+    for (int w = 0; w < SQ_THREADS / 32; ++w) v[w] = red[w][c];
+#pragma unroll
+    for (int w = 0; w < SQ_THREADS / 32; ++w) t += v[w];
+    return t;
 }
 
 // Coordinates along one axis of a box, visited in ascending wrapped order.
@@ -162,13 +182,12 @@ static_assert(3 * SQ_SORT_CAP * sizeof(int) <= SQ_BATCH * sizeof(ChgSh), "the ch
 // What one update keeps in shared memory besides the batch stage.
 struct SqShared {
     SqState s;
-    double sums[8];
+    double red[SQ_THREADS / 32][6], sum;
     double mass_delta;            // stored mass that covered and uncovered nodes take or bring (correction steps)
     long long dfluid;
     int total, box[6], rebuild, ncand, few, nins, nrem;
     int wbox[3];                  // the box's corner wrapped into the lattice
-    int ci[3];                    // the centre: the node below it (wrapped) ...
-    float cf[3];                  // ... and the fraction of a cell above that
+    float off[3];                 // the centre from the node below the candidate list's
     typename cub::BlockScan<int, SQ_THREADS>::TempStorage scan;
 };
 
@@ -179,37 +198,35 @@ struct SqShared {
 //  channels here). Everything stays in shared memory, one warp replays the
 //  changes, and the list is edited (entries gained and lost near the changed
 //  nodes) instead of being rebuilt by two walks over the sphere's box.
-//  The update is bound by latency: it runs once per step on one SM, so besides
-//  its dependent loads it waits for its own instructions, which come from a
-//  cold cache (straight-line code cost 140 cycles per 128 bytes of it). Hence
-//  short loops with the tasks spread over the threads, and divisions done once
-//  for all components. Whole update, launched back to back: 14.9 -> 8.3 us
-//  (64x34x32, R = 4), 13.6 -> 8.5 us (128x64x64, R = 6), 21.7 -> 11.3 us
-//  (256x128x128, R = 8); a step with changes 55-68 us before, 15-22 us with
-//  this. Channel step 37.8 -> 28.2 us, slit step 38.9 -> 34.2 us.
+//  The whole update is bound by latency, on one SM: its dependent loads, its
+//  FP64 chains (8 cycles an addition, 130 a division), its barriers and its
+//  instruction fetches. Hence reads gathered into one round, ordered sums over
+//  values already in registers, divisions done once for all components, and
+//  the velocity set from immediates. Launched back to back the update takes
+//  7.1 us (64x34x32, R = 4; 14.9 with rebuilt lists and serial parts) to 9.1 us
+//  (256x128x128, R = 8; 21.7); a step with changes adds about 4-6 us (before:
+//  35-45 us). 64x34x32 FP64 channel: 37.7 -> 20.3 us a step.
 // ---------------------------------------------------------------------------
 struct FewSh {
-    double pop[SQ_FEW][Q];        // covered: the node's stored numbers; uncovered: the refilled ones
-    double nbrho[SQ_FEW][Q];
+    double pop[SQ_FEW][Q];        // covered: the node's stored numbers
+    double nbrho[SQ_FEW][Q];      // uncovered: the neighbours' densities
     double part[SQ_FEW][6];       // what the change adds to Fc, Tc
-    double r[SQ_FEW][3], ub[SQ_FEW][3], rr[SQ_FEW], mass[SQ_FEW];
+    double ub[SQ_FEW][3], rr[SQ_FEW], mass[SQ_FEW];
     unsigned fnode[SQ_FEW];       // changed nodes as found
-    int fx[SQ_FEW], fy[SQ_FEW], fz[SQ_FEW], fkind[SQ_FEW], fkey[SQ_FEW];
+    int fkind[SQ_FEW];
     unsigned node[SQ_FEW];        // in the order of their first visit in the box
     int x[SQ_FEW], y[SQ_FEW], z[SQ_FEW], kind[SQ_FEW];   // kind: 1 covered, 2 uncovered
-    int nbord[SQ_FEW][Q];         // the change that neighbour j is, or -1
+    int8_t nbord[SQ_FEW][Q];      // the change that neighbour j is, or -1
     uint8_t flag[SQ_FEW][Q];      // flag byte of neighbour j (0: the node) before the changes
     uint8_t near[SQ_FEW][Q];      // neighbour j (0: the node) has a PARTICLE neighbour after them
     unsigned ins[SQ_FEW * Q], rem[SQ_FEW * Q];           // nodes that enter / leave the link list
-    int list[SQ_FEW_LINKS];
+    int list[SQ_FEW_LINKS];       // the link list (fetched ahead)
 };
-// The candidates fetched ahead, each written and read by the same thread (in
-// registers they took the update to 128 a thread and spills).
+// The candidates fetched ahead, each written and read by the same thread: the
+// node, and its offset from the node below the list's reference centre, 10 bits
+// an axis (R <= 200), with its type.
 struct CandSh {
-    unsigned n[SQ_PRE * SQ_THREADS];
-    int x[SQ_PRE * SQ_THREADS];
-    unsigned yz[SQ_PRE * SQ_THREADS];   // y, z < 65536
-    uint8_t ty[SQ_PRE * SQ_THREADS];
+    unsigned n[SQ_PRE * SQ_THREADS], word[SQ_PRE * SQ_THREADS];
 };
 constexpr size_t FEW_BYTES = (sizeof(FewSh) + 15) / 16 * 16;
 static_assert(FEW_BYTES + sizeof(CandSh) <= SQ_BATCH * sizeof(ChgSh),
@@ -227,6 +244,15 @@ __device__ __forceinline__ bool near_or_same(const Lattice& L, const FewSh& w, i
     return dx <= 1 && dy <= 1 && dz <= 1 && dx + dy + dz < 3;
 }
 __device__ __forceinline__ int wrap1(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
+__device__ __forceinline__ unsigned node_at(const Lattice& L, int x, int y, int z) {
+    return (unsigned)x + (unsigned)L.nx * ((unsigned)y + (unsigned)L.ny * (unsigned)z);
+}
+// equilibrium() (lattice.hpp:42-47) of direction i
+__device__ __forceinline__ double equilibrium_rt(int i, double rr, const double* ub) {
+    const double cu = cx_rt(i) * ub[0] + cy_rt(i) * ub[1] + cz_rt(i) * ub[2];
+    const double usq = ub[0] * ub[0] + ub[1] * ub[1] + ub[2] * ub[2];
+    return w_rt(i) * rr * (1.0 + 3.0 * cu + 4.5 * cu * cu - 1.5 * usq);
+}
 
 // Called by all threads; w.f* hold the nfew changes in any order.
 template <class S>
@@ -235,73 +261,84 @@ __device__ __forceinline__ void remap_few(const Lattice& L, const SqArgs& a, SqS
     SqState& s = sh.s;
     const int tid = threadIdx.x;
     const int nold = s.n_links;
-#pragma unroll 1
-    for (int k = tid; k < nold; k += SQ_THREADS) w.list[k] = a.links[k];
-    if (tid < nfew) {   // order of the first visit in the box: rank on the visit index
-        const int key = w.fkey[tid];
+    if (tid < 32) {   // order of the first visit in the box (z, y, x): rank on the visit index
+        const unsigned n = tid < nfew ? w.fnode[tid] : 0u, q = n / (unsigned)L.nx, z = q / (unsigned)L.ny;
+        const int x = (int)(n - q * (unsigned)L.nx), y = (int)(q - z * (unsigned)L.ny);
+        const int kx = x - sh.wbox[0], ky = y - sh.wbox[1], kz = (int)z - sh.wbox[2];
+        const int key = ((kz < 0 ? kz + L.nz : kz) * sh.box[4] + (ky < 0 ? ky + L.ny : ky)) * sh.box[3] +
+                        (kx < 0 ? kx + L.nx : kx);
         int rank = 0;
 #pragma unroll 1
-        for (int j = 0; j < nfew; ++j) rank += w.fkey[j] < key;
-        w.node[rank] = w.fnode[tid]; w.x[rank] = w.fx[tid]; w.y[rank] = w.fy[tid]; w.z[rank] = w.fz[tid];
-        w.kind[rank] = w.fkind[tid];
+        for (int j = 0; j < nfew; ++j) rank += __shfl_sync(0xffffffffu, key, j) < key;
+        if (tid < nfew) {
+            w.node[rank] = n;
+            w.x[rank] = x; w.y[rank] = y; w.z[rank] = (int)z;
+            w.kind[rank] = w.fkind[tid];
+        }
     }
+    for (int k = tid; k < nfew * Q; k += SQ_THREADS) w.near[k / Q][k % Q] = 0;
     __syncthreads();
     // Everything that is read, in one round: the flags of the changed nodes
     // and their neighbours, a covered node's populations, an uncovered one's
-    // neighbouring densities ...
+    // neighbouring densities (tasks below nfew Q), and for each of those nodes
+    // whether one of its 18 neighbours is PARTICLE once the changes are made
+    // (a changed node's type follows from its kind).
 #pragma unroll 1
-    for (int q = tid; q < nfew * Q; q += SQ_THREADS) {
-        const int e = q / Q, j = q - e * Q;
-        const int x = w.x[e], y = w.y[e], z = w.z[e], kind = w.kind[e];
-        const unsigned m = nbr_rt(L, x, y, z, c_cx[j], c_cy[j], c_cz[j]);
-        w.flag[e][j] = a.flag[m];
-        if (kind == 1) w.pop[e][j] = Pop<S>::raw(a.f, logical_slot(L, a.parity, j, w.node[e], x, y, z));
-        else w.nbrho[e][j] = a.rho[m];
+    for (int q = tid; q < nfew * Q * Q; q += SQ_THREADS) {
+        const bool near = q >= nfew * Q;
+        const int ej = near ? (q - nfew * Q) / 18 : q, i = near ? (q - nfew * Q) % 18 + 1 : 0;
+        const int e = ej / Q, j = ej - e * Q;
+        int x = wrap1(w.x[e] + cx_rt(j), L.nx), y = wrap1(w.y[e] + cy_rt(j), L.ny), z = wrap1(w.z[e] + cz_rt(j), L.nz);
+        if (near) { x = wrap1(x + cx_rt(i), L.nx); y = wrap1(y + cy_rt(i), L.ny); z = wrap1(z + cz_rt(i), L.nz); }
+        const unsigned m = node_at(L, x, y, z);
+        const uint8_t fm = a.flag[m];
+        double v = 0.0;
+        if (!near)
+            v = w.kind[e] == 1 ? Pop<S>::raw(a.f, logical_slot(L, a.parity, j, w.node[e], w.x[e], w.y[e], w.z[e])) : a.rho[m];
         int o = -1;
 #pragma unroll 1
         for (int k = 0; k < nfew; ++k)
             if (w.node[k] == m) o = k;
-        w.nbord[e][j] = o;
-        w.near[e][j] = 0;
+        if (near) {
+            if (o >= 0 ? w.kind[o] == 1 : (fm & TYPE_MASK) == T_PARTICLE) w.near[e][j] = 1;
+        } else {
+            w.flag[e][j] = fm;
+            w.nbord[e][j] = (int8_t)o;
+            (w.kind[e] == 1 ? w.pop : w.nbrho)[e][j] = v;
+        }
     }
     __syncthreads();
-    // ... and for each of those nodes whether one of its 18 neighbours is
-    // PARTICLE once the changes are made (a changed node's type follows from
-    // its kind).
-#pragma unroll 1
-    for (int q = tid; q < nfew * Q * 18; q += SQ_THREADS) {
-        const int ej = q / 18, i = q - ej * 18 + 1;
-        const int e = ej / Q, j = ej - e * Q;
-        const int x = wrap1(w.x[e] + c_cx[j], L.nx), y = wrap1(w.y[e] + c_cy[j], L.ny), z = wrap1(w.z[e] + c_cz[j], L.nz);
-        const unsigned m = nbr_rt(L, x, y, z, c_cx[i], c_cy[i], c_cz[i]);
-        bool particle = (a.flag[m] & TYPE_MASK) == T_PARTICLE;
-#pragma unroll 1
-        for (int k = 0; k < nfew; ++k)
-            if (w.node[k] == m) particle = w.kind[k] == 1;
-        if (particle) w.near[e][j] = 1;
-    }
     if (tid < 32) {   // lane e replays change e; an uncovered node waits for the refills it reads
         const int e = tid;
         const bool mine = e < nfew;
         const int kind = mine ? w.kind[e] : 0;
-        double r[3] = {0, 0, 0}, p[3] = {0, 0, 0};
-        unsigned dep = 0;
+        double r[3] = {0, 0, 0}, p[3] = {0, 0, 0}, nb[Q];
+        unsigned dep = 0, fluid = 0;
         if (mine) offset_from_squirmer(L, &s, w.x[e], w.y[e], w.z[e], r);
         if (kind == 1) {   // covered: momentum of the node's populations (lbm.cpp:294-298)
             double m = 0;
-#pragma unroll 1
+#pragma unroll
+            for (int i = 0; i < Q; ++i) nb[i] = w.pop[e][i];
+#pragma unroll
             for (int i = 0; i < Q; ++i) {
-                const double raw = w.pop[e][i];
-                const double fv = S::shifted ? c_w[i] + raw : raw;
-                p[0] += fv * c_cx[i]; p[1] += fv * c_cy[i]; p[2] += fv * c_cz[i];
-                m += raw;
+                const double fv = S::shifted ? WD(i) + nb[i] : nb[i];
+                if (CX(i) > 0) p[0] += fv; else if (CX(i) < 0) p[0] -= fv;
+                if (CY(i) > 0) p[1] += fv; else if (CY(i) < 0) p[1] -= fv;
+                if (CZ(i) > 0) p[2] += fv; else if (CZ(i) < 0) p[2] -= fv;
+                m += nb[i];
             }
             w.mass[e] = m;
         } else if (kind == 2) {
-#pragma unroll 1
+#pragma unroll
             for (int j = 1; j < Q; ++j) {
                 const int o = w.nbord[e][j];
-                if (o >= 0 && o < e && w.kind[o] == 2) dep |= 1u << o;
+                bool fl = (w.flag[e][j] & TYPE_MASK) == T_FLUID;
+                nb[j] = w.nbrho[e][j];
+                if (o >= 0 && o < e) {   // changed earlier
+                    fl = w.kind[o] == 2;
+                    if (fl) dep |= 1u << o;
+                }
+                if (fl) fluid |= 1u << j;
             }
         }
         bool done = kind != 2;
@@ -309,29 +346,22 @@ __device__ __forceinline__ void remap_few(const Lattice& L, const SqArgs& a, SqS
         for (unsigned all = __ballot_sync(0xffffffffu, done); all != 0xffffffffu;) {
             if (!done && (dep & ~all) == 0) {   // uncovered: refill (lbm.cpp:302-317)
                 double rs = 0;
-                int cntf = 0;
-#pragma unroll 1
-                for (int j = 1; j < Q; ++j) {
-                    const int o = w.nbord[e][j];
-                    uint8_t ty = w.flag[e][j] & TYPE_MASK;
-                    double rv = w.nbrho[e][j];
-                    if (o >= 0 && o < e) {   // changed earlier
-                        ty = w.kind[o] == 1 ? T_PARTICLE : T_FLUID;
-                        if (w.kind[o] == 2) rv = w.rr[o];
+                if (dep)
+                    for (int j = 1; j < Q; ++j) {   // a refilled neighbour's density
+                        const int o = w.nbord[e][j];
+                        if (o >= 0 && o < e && w.kind[o] == 2) w.nbrho[e][j] = w.rr[o];
                     }
-                    if (ty == T_FLUID) { rs += rv; ++cntf; }
+#pragma unroll
+                for (int j = 1; j < Q; ++j) {
+                    const double v = dep ? w.nbrho[e][j] : nb[j];
+                    if (fluid >> j & 1u) rs += v;
                 }
-                const double rr = cntf ? rs / cntf : 1.0;
+                const double rr = fluid ? rs / __popc(fluid) : 1.0;
                 double ub[3];
                 surface_velocity(&s, r, ub, false);
                 w.rr[e] = rr;
+#pragma unroll
                 for (int d = 0; d < 3; ++d) { w.ub[e][d] = ub[d]; p[d] = rr * ub[d]; }
-                const double usq = ub[0] * ub[0] + ub[1] * ub[1] + ub[2] * ub[2];
-#pragma unroll 1
-                for (int i = 0; i < Q; ++i) {   // equilibrium() (lattice.hpp:42-47) at (rr, U + W x r)
-                    const double cu = c_cx[i] * ub[0] + c_cy[i] * ub[1] + c_cz[i] * ub[2];
-                    w.pop[e][i] = c_w[i] * rr * (1.0 + 3.0 * cu + 4.5 * cu * cu - 1.5 * usq);
-                }
                 done = true;
             }
             __syncwarp();
@@ -353,55 +383,59 @@ __device__ __forceinline__ void remap_few(const Lattice& L, const SqArgs& a, SqS
             *acc = v;
         }
         if (tid == 0) {
-            sh.nins = sh.nrem = 0;
             sh.dfluid += 2 * __popc(unc) - nfew;
             if (corr_step) {
                 double md = sh.mass_delta;
                 for (int k = 0; k < nfew; ++k) {
                     if (w.kind[k] == 1) md -= w.mass[k];
                     else
-                        for (int i = 0; i < Q; ++i) md += Pop<S>::stored_raw(w.pop[k][i], i);
+                        for (int i = 0; i < Q; ++i) md += Pop<S>::stored_raw(equilibrium_rt(i, w.rr[k], w.ub[k]), i);
                 }
                 sh.mass_delta = md;
             }
         }
+    } else {
+        // Meanwhile the nodes' new types, and the nodes that enter or leave the
+        // link list: only the changed nodes and their neighbours can, each
+        // handled once, by the first change it is near.
+#pragma unroll 1
+        for (int q = tid - 32; q < nfew * Q; q += SQ_THREADS - 32) {
+            const int e = q / Q, j = q - e * Q;
+            const int x = wrap1(w.x[e] + cx_rt(j), L.nx), y = wrap1(w.y[e] + cy_rt(j), L.ny),
+                      z = wrap1(w.z[e] + cz_rt(j), L.nz);
+            bool first = true;
+#pragma unroll 1
+            for (int k = 0; k < e; ++k) first = first && !near_or_same(L, w, k, x, y, z);
+            if (!first) continue;
+            const unsigned m = node_at(L, x, y, z);
+            const int o = w.nbord[e][j];   // the change that m is
+            const uint8_t fm = w.flag[e][j];
+            uint8_t nf = fm & (uint8_t)~NEAR_PARTICLE;
+            if (o >= 0) {
+                const bool nw = (L.walls_y && (y == 1 || y == L.ny - 2)) || (L.walls_z && (z == 1 || z == L.nz - 2));
+                nf = w.kind[o] == 1 ? T_PARTICLE : (uint8_t)(T_FLUID | (nw ? NEAR_WALL : 0));
+            }
+            const bool was = (fm & NEAR_PARTICLE) != 0, is = (nf & TYPE_MASK) == T_FLUID && w.near[e][j];
+            if (is) nf |= NEAR_PARTICLE;
+            if (nf != fm) a.flag[m] = nf;
+            if (is && !was) w.ins[atomicAdd(&sh.nins, 1)] = m;
+            if (was && !is) w.rem[atomicAdd(&sh.nrem, 1)] = m;
+        }
     }
     __syncthreads();
-    // Scatter: types, refilled populations, rho/u of uncovered nodes; and the
-    // nodes that enter or leave the link list: only the changed nodes and
-    // their neighbours can, each handled once, by the first change it is near.
+    // the refilled populations, rho and u of uncovered nodes
 #pragma unroll 1
     for (int q = tid; q < nfew * Q; q += SQ_THREADS) {
         const int e = q / Q, j = q - e * Q;
+        if (w.kind[e] != 2) continue;
         const unsigned n = w.node[e];
-        if (w.kind[e] == 2) {
-            Pop<S>::put(a.f, logical_slot(L, a.parity, j, n, w.x[e], w.y[e], w.z[e]), j, w.pop[e][j]);
-            if (j == 0) { a.rho[n] = w.rr[e]; a.ux[n] = w.ub[e][0]; a.uy[n] = w.ub[e][1]; a.uz[n] = w.ub[e][2]; }
-        }
-        const int x = wrap1(w.x[e] + c_cx[j], L.nx), y = wrap1(w.y[e] + c_cy[j], L.ny), z = wrap1(w.z[e] + c_cz[j], L.nz);
-        bool first = true;
-#pragma unroll 1
-        for (int k = 0; k < e; ++k) first = first && !near_or_same(L, w, k, x, y, z);
-        if (!first) continue;
-        const unsigned m = (unsigned)x + (unsigned)L.nx * ((unsigned)y + (unsigned)L.ny * (unsigned)z);
-        const int o = w.nbord[e][j];   // the change that m is
-        const uint8_t fm = w.flag[e][j];
-        uint8_t nf = fm & (uint8_t)~NEAR_PARTICLE;
-        if (o >= 0) {
-            const bool nw = (L.walls_y && (y == 1 || y == L.ny - 2)) || (L.walls_z && (z == 1 || z == L.nz - 2));
-            nf = w.kind[o] == 1 ? T_PARTICLE : (uint8_t)(T_FLUID | (nw ? NEAR_WALL : 0));
-        }
-        const bool was = (fm & NEAR_PARTICLE) != 0, is = (nf & TYPE_MASK) == T_FLUID && w.near[e][j];
-        if (is) nf |= NEAR_PARTICLE;
-        if (nf != fm) a.flag[m] = nf;
-        if (is && !was) w.ins[atomicAdd(&sh.nins, 1)] = m;
-        if (was && !is) w.rem[atomicAdd(&sh.nrem, 1)] = m;
+        Pop<S>::put(a.f, logical_slot(L, a.parity, j, n, w.x[e], w.y[e], w.z[e]), j, equilibrium_rt(j, w.rr[e], w.ub[e]));
+        if (j == 0) { a.rho[n] = w.rr[e]; a.ux[n] = w.ub[e][0]; a.uy[n] = w.ub[e][1]; a.uz[n] = w.ub[e][2]; }
     }
-    __syncthreads();
     const int nins = sh.nins, nrem = sh.nrem;
     if (nins + nrem > 0) {   // uniform: every entry to its new place in the ascending list
 #pragma unroll 1
-        for (int k = tid; k < nold + nins; k += SQ_THREADS) {
+        for (int k = SQ_THREADS - 1 - tid; k < nold + nins; k += SQ_THREADS) {
             const bool fresh = k >= nold;
             const unsigned n = fresh ? w.ins[k - nold] : (unsigned)w.list[k];
             int pos = k;
@@ -631,7 +665,7 @@ __device__ __noinline__ void remap_walk(const Lattice& L, const SqArgs& a, SqSha
                 for (int i = 0; i < Q; ++i) {
                     const size_t k = logical_slot(L, a.parity, i, n, x, y, z);
                     const double fv = Pop<S>::get(a.f, k, i);
-                    p0 += fv * c_cx[i]; p1 += fv * c_cy[i]; p2 += fv * c_cz[i];
+                    p0 += fv * cx_rt(i); p1 += fv * cy_rt(i); p2 += fv * cz_rt(i);
                     m += Pop<S>::raw(a.f, k);
                 }
                 c.p[0] = p0; c.p[1] = p1; c.p[2] = p2; c.mass = m;
@@ -646,8 +680,8 @@ __device__ __noinline__ void remap_walk(const Lattice& L, const SqArgs& a, SqSha
             const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
                       z = (int)(n / L.nxy);
             // lbm.cpp:305: neighbour with wrap in every axis
-            const int xn = (x + c_cx[j] + L.nx) % L.nx, yn = (y + c_cy[j] + L.ny) % L.ny,
-                      zn = (z + c_cz[j] + L.nz) % L.nz;
+            const int xn = (x + cx_rt(j) + L.nx) % L.nx, yn = (y + cy_rt(j) + L.ny) % L.ny,
+                      zn = (z + cz_rt(j) + L.nz) % L.nz;
             const unsigned m = (unsigned)xn + (unsigned)L.nx * ((unsigned)yn + (unsigned)L.ny * (unsigned)zn);
             c.nbfl[j - 1] = a.flag[m] & TYPE_MASK;
             c.nbrho[j - 1] = a.rho[m];
@@ -697,8 +731,8 @@ __device__ __noinline__ void remap_walk(const Lattice& L, const SqArgs& a, SqSha
                 if (corr_step) {
                     const double usq = ub[0] * ub[0] + ub[1] * ub[1] + ub[2] * ub[2];
                     for (int i = 0; i < Q; ++i) {
-                        const double cu = c_cx[i] * ub[0] + c_cy[i] * ub[1] + c_cz[i] * ub[2];
-                        const double feq = c_w[i] * rr * (1.0 + 3.0 * cu + 4.5 * cu * cu - 1.5 * usq);
+                        const double cu = cx_rt(i) * ub[0] + cy_rt(i) * ub[1] + cz_rt(i) * ub[2];
+                        const double feq = w_rt(i) * rr * (1.0 + 3.0 * cu + 4.5 * cu * cu - 1.5 * usq);
                         sh_mass_delta += Pop<S>::stored_raw(feq, i);
                     }
                 }
@@ -723,9 +757,9 @@ __device__ __noinline__ void remap_walk(const Lattice& L, const SqArgs& a, SqSha
             }
             if (c.kind == 2) {
                 // equilibrium() (lattice.hpp:42-47) at (rr, U + W x r)
-                const double cu = c_cx[i] * c.ub[0] + c_cy[i] * c.ub[1] + c_cz[i] * c.ub[2];
+                const double cu = cx_rt(i) * c.ub[0] + cy_rt(i) * c.ub[1] + cz_rt(i) * c.ub[2];
                 const double usq = c.ub[0] * c.ub[0] + c.ub[1] * c.ub[1] + c.ub[2] * c.ub[2];
-                const double feq = c_w[i] * c.rr * (1.0 + 3.0 * cu + 4.5 * cu * cu - 1.5 * usq);
+                const double feq = w_rt(i) * c.rr * (1.0 + 3.0 * cu + 4.5 * cu * cu - 1.5 * usq);
                 Pop<S>::put(a.f, logical_slot(L, a.parity, i, n, x, y, z), i, feq);
             }
         }
@@ -833,216 +867,256 @@ __device__ __forceinline__ void store_sq_state(SqState* dst, const SqState& s) {
     if (t == ST && s.status) atomicOr(&dst->status, s.status);
 }
 
-// The rigid body (stage BODY), the sphere's box and what the remap's test needs
-// of the new centre. Warp 0 holds the components of X and U in its lanes 0-2,
-// warp 1 those of W and e, so that each division (most of the instructions
-// here) runs once for all components and the two chains side by side. The
-// values are the reference's, operation for operation.
-__device__ __forceinline__ void body_rotation(SqShared& sh) {   // warp 1
+// a / b, correctly rounded, given y = 1 / b correctly rounded (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990): the residual of a y is exact in one FMA and the corrected quotient
+// rounds as the division does. Outside the range where the residual is exact
+// (and for zero, infinite or NaN operands) the division itself decides.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    const double q = a * y;
+    if (!(fabs(q) > 1e-280 && fabs(q) < 1e280 && fabs(a) > 1e-280 && fabs(a) < 1e280)) return a / b;
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+// The rigid body (stage BODY) and what the remap's test needs of the new
+// centre. Warp 0 holds the components of X and U in its lanes 0-2, warp 1
+// those of W and e: each step of the two chains runs once for all components,
+// and side by side. What does not depend on the force is fetched and formed
+// before the wait (BodyPre). The values are the reference's, operation for
+// operation.
+struct BodyPre {
+    double X, v, c, M, y;         // component d: X, U, Fc, M, 1/M (warp 0); e, W, Tc, I, 1/I (warp 1)
+    double e1, e2;                // warp 1: e[d + 1], e[d + 2]
+    double lo, hi, Xs;            // warp 0: the hard gap's bounds, the node below the list's centre
+    double R, hc, base;           // base: the list's centre
+    int planar;
+};
+__device__ __forceinline__ BodyPre body_pre(const Lattice& L, const SqState& s, const double* shell_X, int warp, int d) {
+    BodyPre b;
+    const int nd = d == 0 ? L.nx : (d == 1 ? L.ny : L.nz), d1 = d == 2 ? 0 : d + 1, d2 = d == 0 ? 2 : d - 1;
+    b.planar = s.planar;
+    b.R = s.R; b.hc = s.hc;
+    b.X = warp == 0 ? s.X[d] : s.e[d];
+    b.v = warp == 0 ? s.U[d] : s.W[d];
+    b.c = warp == 0 ? s.Fc[d] : s.Tc[d];
+    b.M = warp == 0 ? s.M : s.I;
+    b.y = 1.0 / b.M;
+    b.e1 = s.e[d1]; b.e2 = s.e[d2];
+    b.lo = 0.5 + s.R + s.hmin; b.hi = (nd - 1.5) - s.R - s.hmin;
+    b.base = d == 0 ? shell_X[0] : (d == 1 ? shell_X[1] : shell_X[2]);
+    b.Xs = floor(b.base);
+    return b;
+}
+__device__ __forceinline__ void body_rotation(SqShared& sh, const BodyPre& b, double T, int lane, int d) {   // warp 1
     SqState& s = sh.s;
     constexpr unsigned ALL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, d = lane < 3 ? lane : 0, d1 = d == 2 ? 0 : d + 1, d2 = d == 0 ? 2 : d - 1;
+    const int d1 = d == 2 ? 0 : d + 1, d2 = d == 0 ? 2 : d - 1;
     // Squirmer::integrate (squirmer.cpp:52-68)
-    double w = s.W[d] + (s.Th[d] + s.Tc[d]) / s.I, e = s.e[d];
-    if (s.planar && d != 2) w = 0.0;
-    e += __shfl_sync(ALL, w, d1) * s.e[d2] - __shfl_sync(ALL, w, d2) * s.e[d1];
-    if (s.planar && d == 2) e = 0.0;
+    double w = b.v + div_by(T + b.c, b.M, b.y), e = b.X;
+    if (b.planar && d != 2) w = 0.0;
+    e += __shfl_sync(ALL, w, d1) * b.e2 - __shfl_sync(ALL, w, d2) * b.e1;
+    if (b.planar && d == 2) e = 0.0;
     const double f0 = __shfl_sync(ALL, e, 0), f1 = __shfl_sync(ALL, e, 1), f2 = __shfl_sync(ALL, e, 2);
     e /= sqrt(f0 * f0 + f1 * f1 + f2 * f2);
-    const bool bad = !(isfinite(w) && isfinite(e) && isfinite(s.Th[d]));
-    __syncwarp();   // every lane has read the old state
-    if (lane < 3) { s.W[d] = w; s.e[d] = e; s.Tc[d] = 0.0; }
-    if (__any_sync(ALL, bad) && lane == 0) atomicOr(&s.status, ST_NAN);
+    if (lane < 3) {
+        s.W[d] = w; s.e[d] = e; s.Tc[d] = 0.0;
+        if (!(isfinite(w) && isfinite(e) && isfinite(T))) atomicOr(&s.status, ST_NAN);
+    }
 }
-__device__ __forceinline__ void body_and_box(const Lattice& L, SqShared& sh, bool body, int shell_ok,
-                                             const double* shell_X) {   // warp 0
+__device__ __forceinline__ void body_motion(const Lattice& L, SqShared& sh, const BodyPre& b, double F, bool body,
+                                            int shell_ok, int lane, int d) {   // warp 0
     SqState& s = sh.s;
     constexpr unsigned ALL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, d = lane < 3 ? lane : 0;
-    const bool lin = lane < 3;
-    const int nd = d == 0 ? L.nx : (d == 1 ? L.ny : L.nz);
     const bool walled = d == 1 ? L.walls_y != 0 : (d == 2 && L.walls_z != 0);
-    double X = s.X[d];
-    bool bad = false, far = false;
+    double X = b.X;
     if (body) {
         // LBM::applyWallPotential (lbm.cpp:231-241): the lower and the upper wall
         double Fw = 0.0;
-        const double hl = X - s.R - 0.5, hu = (nd - 1.5) - X - s.R;
-        if (walled && hl < s.hc) Fw += soft_wall_force(hl, s.eps, s.FS, s.hc);
-        if (walled && hu < s.hc) Fw -= soft_wall_force(hu, s.eps, s.FS, s.hc);
+        if (walled) {
+            const int nd = d == 1 ? L.ny : L.nz;
+            const double hl = X - b.R - 0.5, hu = (nd - 1.5) - X - b.R;
+            if (hl < b.hc) Fw += soft_wall_force(hl, s.eps, s.FS, b.hc);
+            if (hu < b.hc) Fw -= soft_wall_force(hu, s.eps, s.FS, b.hc);
+        }
         // Squirmer::integrate (squirmer.cpp:52-68)
-        double v = s.U[d] + (s.Fh[d] + s.Fc[d] + Fw) / s.M;
-        if (s.planar && d == 2) v = 0.0;
-        const double Xold = X;
+        double v = b.v + div_by(F + b.c + Fw, b.M, b.y);
+        if (b.planar && d == 2) v = 0.0;
         X += v;
-        // LBM::enforceMinimumGap (lbm.cpp:245-253)
-        bool hitl = false, hith = false;
-        if (lin && walled) {
-            const double lo = 0.5 + s.R + s.hmin, hi = (nd - 1.5) - s.R - s.hmin;
-            if (X < lo) { X = lo; if (v < 0) v = 0; hitl = true; }
-            if (X > hi) { X = hi; if (v > 0) v = 0; hith = true; }
+        int hits = 0;
+        if (walled) {   // LBM::enforceMinimumGap (lbm.cpp:245-253)
+            if (X < b.lo) { X = b.lo; if (v < 0) v = 0; ++hits; }
+            if (X > b.hi) { X = b.hi; if (v > 0) v = 0; ++hits; }
         }
-        bad = __any_sync(ALL, !(isfinite(X) && isfinite(v) && isfinite(s.Fh[d])));
-        // The densities the refill reads were stored for the box of the
-        // previous position widened by 2; that covers this step's box
-        // widened by 1 only if the centre moved less than one cell.
-        far = __any_sync(ALL, fabs(X - Xold) >= 1.0) && !bad;
-        const int hits = __popc(__ballot_sync(ALL, hitl)) + __popc(__ballot_sync(ALL, hith));
-        if (lin) { s.X[d] = X; s.U[d] = v; s.Fw[d] = Fw; s.Fc[d] = 0.0; }
-        if (lane == 0) {
-            s.t += 1;
-            s.contacts += hits;
-            if (bad || far) atomicOr(&s.status, bad ? ST_NAN : ST_REMAP_RANGE);
+        if (lane < 3) {
+            s.X[d] = X; s.U[d] = v; s.Fw[d] = Fw; s.Fc[d] = 0.0;
+            // The densities the refill reads were stored for the box of the
+            // previous position widened by 2; that covers this step's box
+            // widened by 1 only if the centre moved less than one cell.
+            if (!(isfinite(X) && isfinite(v) && isfinite(F))) atomicOr(&s.status, ST_NAN);
+            else if (fabs(X - b.X) >= 1.0) atomicOr(&s.status, ST_REMAP_RANGE);
+            if (hits) atomicAdd(reinterpret_cast<unsigned long long*>(&s.contacts), (unsigned long long)hits);
+            if (d == 0) s.t += 1;
         }
     }
-    if (lin && !bad && !far) {
-        // the sphere's bounding box (lbm.cpp:272-276)
-        int b0 = (int)floor(X - s.R) - 2, b1 = (int)ceil(X + s.R) + 2;
-        if (d == 1 && walled) { b0 = max(0, b0); b1 = min(nd - 1, b1); }
-        sh.box[d] = b0;
-        sh.box[3 + d] = b1 - b0 + 1;
-        // the centre as a node index and a fraction of a cell, for the FP32 test
-        const double c0 = floor(X);
-        sh.cf[d] = (float)(X - c0);
-        double ci = c0;
-        if (!walled && !(c0 >= 0.0 && c0 < nd)) ci -= nd * floor(c0 / nd);
-        sh.ci[d] = (int)ci;
-        sh.wbox[d] = b0 >= 0 && b0 < nd ? b0 : ((b0 % nd) + nd) % nd;
-    }
-    const double q = X - shell_X[d];
-    const double q0 = __shfl_sync(ALL, q, 0), q1 = __shfl_sync(ALL, q, 1), q2 = __shfl_sync(ALL, q, 2);
-    if (lane == 0) sh.rebuild = !(shell_ok && q0 * q0 + q1 * q1 + q2 * q2 < SHELL_SLACK * SHELL_SLACK);
+    const double q = X - b.base, q2 = q * q;
+    const double r2 = __shfl_sync(ALL, q2, 0) + __shfl_sync(ALL, q2, 1) + __shfl_sync(ALL, q2, 2);
+    if (lane == 0) sh.rebuild = !(shell_ok && r2 < SHELL_SLACK * SHELL_SLACK);
+    if (lane < 3) sh.off[d] = (float)(X - b.Xs);
+}
+// The sphere's bounding box (lbm.cpp:272-276) and the zones of the coming steps
+// around it (see ZoneBox), beside the remap's test: lane d of one warp.
+__device__ __forceinline__ void box_and_zones(const Lattice& L, const SqArgs& a, SqShared& sh, int d) {
+    SqState& s = sh.s;
+    const int nd = d == 0 ? L.nx : (d == 1 ? L.ny : L.nz);
+    const bool walled = d == 1 ? L.walls_y != 0 : (d == 2 && L.walls_z != 0);
+    int b0 = (int)floor(s.X[d] - s.R) - 2, b1 = (int)ceil(s.X[d] + s.R) + 2;
+    if (d == 1 && walled) { b0 = max(0, b0); b1 = min(nd - 1, b1); }
+    const int wb = b0 >= 0 && b0 < nd ? b0 : ((b0 % nd) + nd) % nd;
+    sh.box[d] = b0;
+    sh.box[3 + d] = b1 - b0 + 1;
+    sh.wbox[d] = wb;
+    const int wd = zone_width(s.R, nd, walled);
+    int lo;
+    if (walled) zone_axis(b0, nd, wd, true, lo);
+    else lo = wd >= nd ? 0 : wrap1(wb - ZONE_MARGIN, nd);   // zone_axis of the wrapped corner
+    if (a.zslot_a >= 0) { s.zone[a.zslot_a].w[d] = wd; s.zone[a.zslot_a].lo[d] = lo; }
+    if (a.zslot_b >= 0) { s.zone[a.zslot_b].w[d] = wd; s.zone[a.zslot_b].lo[d] = lo; }
 }
 
-template <class S, bool PDL>
-__device__ __forceinline__ void squirmer_update(const Lattice& L, const SqArgs& a) {
+// One update. wait() returns once everything the update reads but its own
+// earlier writes is complete (false: that never came, and the update leaves).
+// early: the state, the candidate list and the node types, which only updates
+// write, may be read before it.
+template <class S, class Wait>
+__device__ __forceinline__ bool squirmer_update(const Lattice& L, const SqArgs& a, bool early, Wait&& wait) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ SqShared sh;
     SqState& s = sh.s;
     const int tid = threadIdx.x;
-    const bool early = PDL && (a.stages & STAGE_PRE) != 0;   // uniform
-    if (PDL && !early) pdl_wait();
+    if (!early && !wait()) return false;
     {   // the state, one word per thread
         constexpr int NS = (int)(sizeof(SqState) / 4);
         static_assert(sizeof(SqState) % 4 == 0 && NS <= SQ_THREADS, "one word per thread");
         if (tid < NS) reinterpret_cast<uint32_t*>(&s)[tid] = __ldcg(reinterpret_cast<const uint32_t*>(a.sq) + tid);
     }
-    // the first candidates of the remap (see stage REMAP), their types and
-    // coordinates, kept in shared memory until the new centre is known
+    // the first candidates of the remap (see stage REMAP) and the link list,
+    // kept in shared memory until the new centre is known
     const bool remap = (a.stages & STAGE_REMAP) != 0;
     int ncand = 0, shell_ok = 0;
     double shell_X[3] = {0, 0, 0};
     CandSh& cs = *reinterpret_cast<CandSh*>(smem_raw + FEW_BYTES);
+    FewSh& fw = *reinterpret_cast<FewSh*>(smem_raw);
+    int cb[3] = {0, 0, 0};   // the node below the list's reference centre, wrapped
+    auto cand_word = [&](unsigned n) {   // offset from cb and type
+        const unsigned q = n / (unsigned)L.nx, z = q / (unsigned)L.ny;
+        int dx = (int)(n - q * (unsigned)L.nx) - cb[0], dy = (int)(q - z * (unsigned)L.ny) - cb[1], dz = (int)z - cb[2];
+        if (2 * dx > L.nx) dx -= L.nx; else if (2 * dx < -L.nx) dx += L.nx;
+        if (!L.walls_y) { if (2 * dy > L.ny) dy -= L.ny; else if (2 * dy < -L.ny) dy += L.ny; }
+        if (!L.walls_z) { if (2 * dz > L.nz) dz -= L.nz; else if (2 * dz < -L.nz) dz += L.nz; }
+        return (unsigned)(dx + 512) << 22 | (unsigned)(dy + 512) << 12 | (unsigned)(dz + 512) << 2 |
+               (unsigned)(__ldcg(a.flag + n) & TYPE_MASK);
+    };
     if (remap) {
         shell_ok = __ldcg(&a.shell_hdr->valid);
         ncand = shell_ok ? __ldcg(&a.shell_hdr->n) : 0;
-        for (int d = 0; d < 3; ++d) shell_X[d] = __ldcg(&a.shell_hdr->X[d]);
+        const int nd[3] = {L.nx, L.walls_y ? 0 : L.ny, L.walls_z ? 0 : L.nz};   // 0: not periodic
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            shell_X[d] = __ldcg(&a.shell_hdr->X[d]);
+            const double c0 = floor(shell_X[d]);
+            cb[d] = (int)(nd[d] && !(c0 >= 0.0 && c0 < nd[d]) ? c0 - nd[d] * floor(c0 / nd[d]) : c0);
+        }
+        const int nl = shell_ok == 2 ? min(__ldcg(&a.sq->n_links), SQ_FEW_LINKS) : 0;
+#pragma unroll 2
+        for (int k = tid; k < nl; k += SQ_THREADS) fw.list[k] = __ldcg(a.links + k);
 #pragma unroll 2
         for (int c = tid; c < min(ncand, SQ_PRE * SQ_THREADS); c += SQ_THREADS) {
             const unsigned n = (unsigned)__ldcg(a.shell + c);
-            cs.ty[c] = __ldcg(a.flag + n) & TYPE_MASK;
-            const unsigned q = n / (unsigned)L.nx, z = q / (unsigned)L.ny;
             cs.n[c] = n;
-            cs.x[c] = (int)(n - q * (unsigned)L.nx);
-            cs.yz[c] = (q - z * (unsigned)L.ny) | z << 16;
+            cs.word[c] = cand_word(n);
         }
     }
     if (tid == 0) {
         sh.mass_delta = 0.0;
         sh.dfluid = 0;
-        sh.few = 0;
+        sh.few = sh.nins = sh.nrem = 0;
         sh.ncand = ncand;
     }
-    if (early) pdl_wait();
-    if (PDL) pdl_launch_dependents();
     __syncthreads();
-    if (s.status & (ST_NAN | ST_REMAP_RANGE | ST_LINK_OVERFLOW)) return;  // invalid already; the host reports it
+    const int warp = tid >> 5, lane = tid & 31, axis = lane < 3 ? lane : 0;
+    BodyPre bp;
+    if (warp < 2) bp = body_pre(L, s, shell_X, warp, axis);
+    if (early && !wait()) return false;
+    if (s.status & (ST_NAN | ST_REMAP_RANGE | ST_LINK_OVERFLOW)) return true;  // invalid already; the host reports it
 
     const bool loop = (a.stages & STAGE_LOOP) != 0;
     const bool corr_step = loop && a.corr_step;
 
     // ---------------- stages FORCE, BODY ----------------
-    if (a.stages & STAGE_FORCE) block_sum_rows<6>(a.link_part, s.n_links, LINK_PART, 0, sh.sums);
-    const bool body = (a.stages & STAGE_BODY) != 0;
-    if (tid < 32) {
-        if ((a.stages & STAGE_FORCE) && tid < 3) s.Fh[tid] = sh.sums[tid];
-        __syncwarp();
-        body_and_box(L, sh, body, shell_ok, shell_X);
-    } else if (tid < 64) {
-        if ((a.stages & STAGE_FORCE) && tid < 35) s.Th[tid - 32] = sh.sums[tid - 29];
-        __syncwarp();
-        if (body) body_rotation(sh);
+    const bool force = (a.stages & STAGE_FORCE) != 0, body = (a.stages & STAGE_BODY) != 0;
+    if (force) {
+        link_warp_sums(a.link_part, s.n_links, (size_t)a.link_cap, sh.red);
+        __syncthreads();
+    }
+    if (warp == 0) {
+        const double F = force ? link_total(sh.red, axis) : s.Fh[axis];
+        if (force && lane < 3) s.Fh[lane] = F;
+        body_motion(L, sh, bp, F, body, shell_ok, lane, axis);
+    } else if (warp == 1) {
+        const double T = force ? link_total(sh.red, 3 + axis) : s.Th[axis];
+        if (force && lane < 3) s.Th[lane] = T;
+        if (body) body_rotation(sh, bp, T, lane, axis);
     }
     __syncthreads();
     if (s.status & (ST_NAN | ST_REMAP_RANGE)) {
         store_sq_state(a.sq, s);
-        return;
+        return true;
     }
 
     // ---------------- stage REMAP ----------------
     // Candidates within the cached shell: each is first tested in FP32 (the
     // squared distance is off by less than 1e-6 R^2 there); one within 1e-5 R^2
-    // + 1e-3 of the surface, or about half a lattice away, by the reference's
-    // FP64 offset. If few nodes change, remap_few does the rest.
+    // + 1e-3 of the surface by the reference's FP64 offset, as is every one in
+    // a lattice hardly wider than the sphere, where the offset may be about
+    // half a lattice. If few nodes change, remap_few does the rest.
     if (remap) {
-        FewSh& w = *reinterpret_cast<FewSh*>(smem_raw);
         bool walk = sh.rebuild != 0;   // uniform
         if (!walk) {
             const double R2 = s.R * s.R;
-            const float R2f = (float)R2, band = 1e-5f * R2f + 1e-3f;
-            const int hx = L.nx - 4, hy = L.walls_y ? 1 << 30 : L.ny - 4, hz = L.walls_z ? 1 << 30 : L.nz - 4;
-#pragma unroll 1
+            const float R2f = (float)R2, span = 2.0f * (float)s.R + 10.0f, ox = sh.off[0], oy = sh.off[1], oz = sh.off[2];
+            const bool tight = L.nx < span || (!L.walls_y && L.ny < span) || (!L.walls_z && L.nz < span);
+            const float band = tight ? 3.0e38f : 1e-5f * R2f + 1e-3f;
+#pragma unroll 2
             for (int c = tid; c < ncand; c += SQ_THREADS) {
-                unsigned n, ty;
-                int x, y, z;
-                if (c < SQ_PRE * SQ_THREADS) {
-                    n = cs.n[c]; ty = cs.ty[c];
-                    x = cs.x[c]; y = (int)(cs.yz[c] & 0xffffu); z = (int)(cs.yz[c] >> 16);
-                } else {
-                    n = (unsigned)a.shell[c]; ty = a.flag[n] & TYPE_MASK;
-                    x = (int)(n % (unsigned)L.nx); y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny); z = (int)(n / L.nxy);
-                }
+                const unsigned wd = c < SQ_PRE * SQ_THREADS ? cs.word[c] : cand_word((unsigned)a.shell[c]);
+                const unsigned ty = wd & 3u;
                 if (ty == T_WALL) continue;
-                int dx = x - sh.ci[0], dy = y - sh.ci[1], dz = z - sh.ci[2];
-                if (2 * dx > L.nx) dx -= L.nx; else if (2 * dx < -L.nx) dx += L.nx;
-                if (!L.walls_y) { if (2 * dy > L.ny) dy -= L.ny; else if (2 * dy < -L.ny) dy += L.ny; }
-                if (!L.walls_z) { if (2 * dz > L.nz) dz -= L.nz; else if (2 * dz < -L.nz) dz += L.nz; }
-                const float ex = (float)dx - sh.cf[0], ey = (float)dy - sh.cf[1], ez = (float)dz - sh.cf[2];
+                const float ex = (float)((int)(wd >> 22) - 512) - ox, ey = (float)((int)(wd >> 12 & 1023u) - 512) - oy,
+                            ez = (float)((int)(wd >> 2 & 1023u) - 512) - oz;
                 const float gap = ex * ex + ey * ey + ez * ez - R2f;
                 bool inside = gap < 0.f;
-                if (fabsf(gap) < band || 2 * abs(dx) > hx || 2 * abs(dy) > hy || 2 * abs(dz) > hz) {
-                    double r[3];
-                    offset_from_squirmer(L, &s, x, y, z, r);
-                    inside = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] < R2;
-                }
+                if (inside == (ty == T_PARTICLE) && fabsf(gap) >= band) continue;
+                const unsigned n = c < SQ_PRE * SQ_THREADS ? cs.n[c] : (unsigned)a.shell[c];
+                const unsigned q = n / (unsigned)L.nx;
+                const int x = (int)(n - q * (unsigned)L.nx), y = (int)(q % (unsigned)L.ny), z = (int)(q / (unsigned)L.ny);
+                double r[3];
+                offset_from_squirmer(L, &s, x, y, z, r);
+                inside = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] < R2;
                 if (inside != (ty == T_PARTICLE)) {
                     const int k = atomicAdd(&sh.few, 1);
                     if (k < SQ_FEW) {
-                        const int kx = x - sh.wbox[0], ky = y - sh.wbox[1], kz = z - sh.wbox[2];
-                        w.fnode[k] = n; w.fx[k] = x; w.fy[k] = y; w.fz[k] = z;
-                        w.fkind[k] = inside ? 1 : 2;
-                        // visit index in the box (z, y, x of the first visit)
-                        w.fkey[k] = ((kz < 0 ? kz + L.nz : kz) * sh.box[4] + (ky < 0 ? ky + L.ny : ky)) * sh.box[3] +
-                                    (kx < 0 ? kx + L.nx : kx);
+                        fw.fnode[k] = n;
+                        fw.fkind[k] = inside ? 1 : 2;
                     }
                 }
             }
         }
-        // meanwhile: the zones of the coming steps, from this box (see ZoneBox)
-        if (tid >= SQ_THREADS - 3) {
-            const int d = SQ_THREADS - 1 - tid, nd = d == 0 ? L.nx : (d == 1 ? L.ny : L.nz);
-            const bool wall_axis = d == 1 ? L.walls_y != 0 : (d == 2 && L.walls_z != 0);
-            const int wd = zone_width(s.R, nd, wall_axis);
-            int lo;
-            zone_axis(sh.box[d], nd, wd, wall_axis, lo);
-            if (a.zslot_a >= 0) { s.zone[a.zslot_a].w[d] = wd; s.zone[a.zslot_a].lo[d] = lo; }
-            if (a.zslot_b >= 0) { s.zone[a.zslot_b].w[d] = wd; s.zone[a.zslot_b].lo[d] = lo; }
-        }
+        if (tid >= SQ_THREADS - 3) box_and_zones(L, a, sh, SQ_THREADS - 1 - tid);
         __syncthreads();
         const int nfew = sh.few;
         walk = walk || (nfew > 0 && (nfew > SQ_FEW || shell_ok != 2 || s.n_links < 0 || s.n_links > SQ_FEW_LINKS));
         if (walk) remap_walk<S>(L, a, sh, smem_raw, shell_ok, corr_step);   // uniform
-        else if (nfew > 0) remap_few<S>(L, a, sh, w, nfew, corr_step);
+        else if (nfew > 0) remap_few<S>(L, a, sh, fw, nfew, corr_step);
         if (tid == 0) s.n_fluid += sh.dfluid;
     }
 
@@ -1050,15 +1124,15 @@ __device__ __forceinline__ void squirmer_update(const Lattice& L, const SqArgs& 
     double mstep = 0.0;
     if (corr_step) {
         __syncthreads();
-        block_sum_rows<1>(a.block_part, a.nblocks, BLOCK_PART, 3, sh.sums);
-        mstep = sh.sums[0];
+        block_sum_rows(a.block_part, a.nblocks, BLOCK_PART, 3, &sh.sum);
+        mstep = sh.sum;
         __syncthreads();
-        block_sum_rows<1>(a.block_part_b, a.nblocks_b, BLOCK_PART, 3, sh.sums);
-        mstep += sh.sums[0];
+        block_sum_rows(a.block_part_b, a.nblocks_b, BLOCK_PART, 3, &sh.sum);
+        mstep += sh.sum;
         if (a.nblocks_w > 0) {
             __syncthreads();
-            block_sum_rows<1>(a.block_part_w, a.nblocks_w, BLOCK_PART, 3, sh.sums);
-            mstep += sh.sums[0];
+            block_sum_rows(a.block_part_w, a.nblocks_w, BLOCK_PART, 3, &sh.sum);
+            mstep += sh.sum;
         }
     }
     if (tid == 0) {
@@ -1087,18 +1161,23 @@ __device__ __forceinline__ void squirmer_update(const Lattice& L, const SqArgs& 
     }
     __syncthreads();
     store_sq_state(a.sq, s);
+    return true;
 }
 
 template <class S>
-__global__ void __launch_bounds__(SQ_THREADS) k_squirmer(const __grid_constant__ Lattice L,
+__global__ void __launch_bounds__(SQ_THREADS, 1) k_squirmer(const __grid_constant__ Lattice L,
                                                          const __grid_constant__ SqArgs a) {
-    squirmer_update<S, true>(L, a);
+    squirmer_update<S>(L, a, (a.stages & STAGE_PRE) != 0, [] {
+        pdl_wait();
+        pdl_launch_dependents();
+        return true;
+    });
 }
 
 // Ensemble: one CTA per member, each with its own lattice and arguments; the
 // per-step settings are the same for all members.
 template <class S>
-__global__ void __launch_bounds__(SQ_THREADS) k_squirmer_batch(const Lattice* lat, const SqArgs* args, SqStep st) {
+__global__ void __launch_bounds__(SQ_THREADS, 1) k_squirmer_batch(const Lattice* lat, const SqArgs* args, SqStep st) {
     __shared__ __align__(16) Lattice L;
     __shared__ __align__(16) SqArgs A;
     {   // the member's records, one word per thread, with this step's settings
@@ -1117,7 +1196,7 @@ __global__ void __launch_bounds__(SQ_THREADS) k_squirmer_batch(const Lattice* la
         }
     }
     __syncthreads();
-    squirmer_update<S, false>(L, A);
+    squirmer_update<S>(L, A, false, [] { return true; });
 }
 
 }  // namespace lbmgpu

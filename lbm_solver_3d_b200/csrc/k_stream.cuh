@@ -1040,8 +1040,8 @@ __device__ __forceinline__ void zone_particle_links(const Lattice& L, const Stre
         const unsigned ns = __shfl_sync(ALL, n, src);
         const double rho = __shfl_sync(ALL, out.rho, src);
         if (on) {
-            const int cx = c_cx[i], cy = c_cy[i], cz = c_cz[i];
-            const double wi = c_w[i];
+            const int cx = cx_rt(i), cy = cy_rt(i), cz = cz_rt(i);
+            const double wi = w_rt(i);
             T* local = f + (size_t)opp_rt(i) * L.N + ns;
             T* remote = f + (size_t)i * L.N + nbr_rt(L, xs, ys, zs, cx, cy, cz);
             double rb[3], ub[3];
@@ -1133,9 +1133,10 @@ __device__ __forceinline__ void zone_cell(const Lattice& L, const StreamArgs& a,
     if (SQ) {
         zone_particle_links<S, PAR>(L, a, sq, n, x, y, z, a.do_mass != 0, w, sums);
         if (active && (fl & NEAR_PARTICLE)) {
-            double* lp = a.link_part + (size_t)a.linkslot[n] * LINK_PART;
-            lp[0] = sums.fp[0]; lp[1] = sums.fp[1]; lp[2] = sums.fp[2];
-            lp[3] = sums.tp[0]; lp[4] = sums.tp[1]; lp[5] = sums.tp[2];
+            double* lp = a.link_part + a.linkslot[n];
+            const size_t cap = (size_t)a.link_cap;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) { lp[d * cap] = sums.fp[d]; lp[(3 + d) * cap] = sums.tp[d]; }
         }
     }
 }

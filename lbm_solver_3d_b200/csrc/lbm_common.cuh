@@ -218,8 +218,9 @@ constexpr int TRAJ_RING = 4096;
 constexpr int TRAJ_COLS = 15;
 
 // Per-node partial sums written by the stream kernel for boundary-link nodes:
-// F (3), T (3), and two spare slots.
-constexpr int LINK_PART = 8;
+// columns F (3), T (3), each of link_cap rows (a warp of the squirmer update
+// reads 32 consecutive rows of a column).
+constexpr int LINK_PART = 6;
 // Per-block partials of the stream kernel on reduction steps: wall force (3), mass (1).
 constexpr int BLOCK_PART = 4;
 
@@ -228,8 +229,9 @@ struct StreamArgs {
     uint8_t* flag;
     double* rho;                  // pre-collision moments (FP64)
     double* ux; double* uy; double* uz;
-    double* link_part;            // [n_links][LINK_PART], one row per near-particle node
+    double* link_part;            // [LINK_PART][link_cap], one row per near-particle node
     const int* linkslot;          // node -> its row of link_part
+    int link_cap;
     double* block_part;           // bulk kernel: [blocks][BLOCK_PART]
     double* block_part_b;         // zone kernel: [blocks][BLOCK_PART]
     const int* wallrows;          // (y, z) of the fluid rows next to a wall

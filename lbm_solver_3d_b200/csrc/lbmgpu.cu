@@ -204,7 +204,7 @@ bool is_corr_step(const lbmgpu_handle* h, long long s) {
 StreamArgs stream_args(lbmgpu_handle* h, const StepPlan& sp) {
     StreamArgs a;
     a.f = h->f; a.flag = h->flag; a.rho = h->rho; a.ux = h->ux; a.uy = h->uy; a.uz = h->uz;
-    a.link_part = h->link_part; a.linkslot = h->linkslot;
+    a.link_part = h->link_part; a.linkslot = h->linkslot; a.link_cap = h->link_cap;
     a.block_part = h->block_part; a.block_part_b = h->block_part_b;
     a.wallrows = h->wallrows; a.n_wallrows = (int)h->geom.nwallrows;
     a.zone_cells = h->zone_cells;
