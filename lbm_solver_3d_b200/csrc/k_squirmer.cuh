@@ -867,17 +867,6 @@ __device__ __forceinline__ void store_sq_state(SqState* dst, const SqState& s) {
     if (t == ST && s.status) atomicOr(&dst->status, s.status);
 }
 
-// a / b, correctly rounded, given y = 1 / b correctly rounded (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor",
-// 1990): the residual of a y is exact in one FMA and the corrected quotient
-// rounds as the division does. Outside the range where the residual is exact
-// (and for zero, infinite or NaN operands) the division itself decides.
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-    const double q = a * y;
-    if (!(fabs(q) > 1e-280 && fabs(q) < 1e280 && fabs(a) > 1e-280 && fabs(a) < 1e280)) return a / b;
-    return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
-
 // The rigid body (stage BODY) and what the remap's test needs of the new
 // centre. Warp 0 holds the components of X and U in its lanes 0-2, warp 1
 // those of W and e: each step of the two chains runs once for all components,
@@ -890,6 +879,7 @@ struct BodyPre {
     double lo, hi, Xs;            // warp 0: the hard gap's bounds, the node below the list's centre
     double R, hc, base;           // base: the list's centre
     int planar;
+    bool yfar;
 };
 __device__ __forceinline__ BodyPre body_pre(const Lattice& L, const SqState& s, const double* shell_X, int warp, int d) {
     BodyPre b;
@@ -901,6 +891,7 @@ __device__ __forceinline__ BodyPre body_pre(const Lattice& L, const SqState& s, 
     b.c = warp == 0 ? s.Fc[d] : s.Tc[d];
     b.M = warp == 0 ? s.M : s.I;
     b.y = 1.0 / b.M;
+    b.yfar = exponent_far(b.M) || b.M == 0.0;
     b.e1 = s.e[d1]; b.e2 = s.e[d2];
     b.lo = 0.5 + s.R + s.hmin; b.hi = (nd - 1.5) - s.R - s.hmin;
     b.base = d == 0 ? shell_X[0] : (d == 1 ? shell_X[1] : shell_X[2]);
@@ -912,7 +903,7 @@ __device__ __forceinline__ void body_rotation(SqShared& sh, const BodyPre& b, do
     constexpr unsigned ALL = 0xffffffffu;
     const int d1 = d == 2 ? 0 : d + 1, d2 = d == 0 ? 2 : d - 1;
     // Squirmer::integrate (squirmer.cpp:52-68)
-    double w = b.v + div_by(T + b.c, b.M, b.y), e = b.X;
+    double w = b.v + div_by(T + b.c, b.M, b.y, exponent_far(T + b.c) || b.yfar), e = b.X;
     if (b.planar && d != 2) w = 0.0;
     e += __shfl_sync(ALL, w, d1) * b.e2 - __shfl_sync(ALL, w, d2) * b.e1;
     if (b.planar && d == 2) e = 0.0;
@@ -939,7 +930,7 @@ __device__ __forceinline__ void body_motion(const Lattice& L, SqShared& sh, cons
             if (hu < b.hc) Fw -= soft_wall_force(hu, s.eps, s.FS, b.hc);
         }
         // Squirmer::integrate (squirmer.cpp:52-68)
-        double v = b.v + div_by(F + b.c + Fw, b.M, b.y);
+        double v = b.v + div_by(F + b.c + Fw, b.M, b.y, exponent_far(F + b.c + Fw) || b.yfar);
         if (b.planar && d == 2) v = 0.0;
         X += v;
         int hits = 0;

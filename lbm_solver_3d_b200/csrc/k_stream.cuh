@@ -226,6 +226,30 @@ struct GlobalSrc {
     }
 };
 
+// a / b, correctly rounded, given y = 1 / b correctly rounded (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990): the residual of a y is exact in one FMA and the corrected quotient
+// rounds as the division does. far: a or b may be outside the range where that
+// holds (see exponent_far), and the division itself decides.
+__device__ __forceinline__ double div_by(double a, double b, double y, bool far) {
+    if (far) return a / b;
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+// not zero and outside 2^-512 .. 2^512 (infinities and NaN included)
+__device__ __forceinline__ bool exponent_far(double a) {
+    const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    return hi - 0x1ff00000u >= 0x40000000u && (hi | (unsigned)__double2loint(a)) != 0u;
+}
+// (a0, a1, a2) / r: one division, the bits of three
+__device__ __forceinline__ void div3(double a0, double a1, double a2, double r, double& u, double& v, double& w) {
+    const double y = 1.0 / r;
+    const bool far = exponent_far(r) || r == 0.0 || exponent_far(a0) || exponent_far(a1) || exponent_far(a2);
+    u = div_by(a0, r, y, far);
+    v = div_by(a1, r, y, far);
+    w = div_by(a2, r, y, far);
+}
+
 // Constants of the collision in the arithmetic A of a storage form (A = float:
 // the FP32 copies kept in Lattice; A = double: the FP64 values themselves).
 template <class A> struct Coll;
@@ -581,7 +605,8 @@ __device__ __forceinline__ void update_node(const Lattice& L, const StreamArgs& 
             if (CZ(i) > 0) mz += fv[i]; else if (CZ(i) < 0) mz -= fv[i];
         }
         const double Fx = L.F[0], Fy = L.F[1], Fz = L.F[2];
-        const double u = (mx + 0.5 * Fx) / r, v = (my + 0.5 * Fy) / r, wz = (mz + 0.5 * Fz) / r;
+        double u, v, wz;
+        div3(mx + 0.5 * Fx, my + 0.5 * Fy, mz + 0.5 * Fz, r, u, v, wz);
         if (store_rho) a.rho[n] = r;
         if (MACRO) { a.ux[n] = u; a.uy[n] = v; a.uz[n] = wz; }
         if (GENERAL) out.rho = r;

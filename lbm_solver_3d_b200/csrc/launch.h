@@ -30,6 +30,7 @@ struct StreamGeom {
 };
 
 struct SqArgs;
+struct ClusterWork;
 
 // device tables of an ensemble
 struct BatchArgs {
@@ -88,6 +89,10 @@ struct Launchers {
     int runs_max_nodes;                // nodes per run
     // one CTA per row (k_bulk_rowcta): rows away from walls, or next to one
     void (*batch_rowcta)(int par, bool macro, bool wallrows, const BatchArgs& b, BatchStep st, cudaStream_t s);
+    // many steps of a small lattice without a squirmer in one cluster (k_cluster_steps): the launch,
+    // and the cluster size that can hold the lattice (0: none), filling rows and stride
+    cudaError_t (*cluster)(const Lattice& L, void* f, const ClusterWork& w, int ctas, cudaStream_t st);
+    int (*cluster_fit)(const Lattice& L, ClusterWork& w);
     size_t esize;
     void (*batch_squirmer)(const BatchArgs& b, SqStep st, cudaStream_t s);
 };

@@ -5,6 +5,7 @@
 #pragma once
 #include "k_aux.cuh"
 #include "k_batch.cuh"
+#include "k_cluster.cuh"
 #include "k_squirmer.cuh"
 #include "k_stream.cuh"
 #include "launch.h"
@@ -301,6 +302,52 @@ static int rows_occupancy(int nx, bool pairs) {
 }
 
 template <class S>
+static cudaLaunchConfig_t cluster_config(const ClusterWork& w, int ctas, cudaLaunchAttribute* at, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(CLUSTER_THREADS);
+    cfg.dynamicSmemBytes = cluster_smem<S>(w.rows, w.stride);
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+template <class S>
+static cudaError_t cluster_launch(const Lattice& L, void* f, const ClusterWork& w, int ctas, cudaStream_t st) {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = cluster_config<S>(w, ctas, at, st);
+    return L.force_free ? cudaLaunchKernelEx(&cfg, k_cluster_steps<S, false>, L, f, w)
+                        : cudaLaunchKernelEx(&cfg, k_cluster_steps<S, true>, L, f, w);
+}
+// The largest cluster of equal parts (whole rows) that holds the lattice and can be resident.
+template <class S>
+static int cluster_fit(const Lattice& L, ClusterWork& w) {
+    constexpr size_t MOST = 227 * 1024;
+    const long long total = (long long)L.ny * L.nz;
+    for (int ctas = CLUSTER_CTAS; ctas >= 8; ctas /= 2) {
+        const long long rows = (total + ctas - 1) / ctas;
+        if (rows * L.nx > CLUSTER_NODES) return 0;
+        w.rows = (int)rows;
+        w.stride = (int)(rows * L.nx + 15) / 16 * 16;
+        const size_t smem = cluster_smem<S>(w.rows, w.stride);
+        if (smem > MOST) return 0;
+        int n = 0;
+        bool ok = true;
+        for (auto fn : {k_cluster_steps<S, false>, k_cluster_steps<S, true>})
+            ok = ok && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                 cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST) == cudaSuccess;
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = cluster_config<S>(w, ctas, at, nullptr);
+        if (ok && cudaOccupancyMaxActiveClusters(&n, k_cluster_steps<S, true>, &cfg) == cudaSuccess && n > 0) return ctas;
+        cudaGetLastError();   // a refused size is not an error of the caller's
+    }
+    return 0;
+}
+
+template <class S>
 static cudaError_t prepare_launch() {
     cudaError_t e = cudaFuncSetAttribute(k_squirmer<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)squirmer_smem());
     if (e != cudaSuccess) return e;
@@ -393,6 +440,8 @@ static Launchers make_launchers() {
     l.chunkp_ctas_per_sm = &chunkp_occupancy<S>;
     l.rows_ctas_per_sm = &rows_occupancy<S>;
     l.batch_runs = &batch_runs_launch<S>;
+    l.cluster = &cluster_launch<S>;
+    l.cluster_fit = &cluster_fit<S>;
     l.runs_max_nodes = RunsCfg<S>::NODES;
     l.esize = sizeof(typename S::T);
     return l;

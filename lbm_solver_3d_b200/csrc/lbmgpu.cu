@@ -36,6 +36,7 @@
 #include "../../include/lbmgpu.h"
 #include "k_aux.cuh"
 #include "k_batch.cuh"
+#include "k_cluster.cuh"
 #include "k_squirmer.cuh"
 #include "launch.h"
 
@@ -101,6 +102,8 @@ struct lbmgpu_handle {
     int zone_cells = 0, zw[3] = {0, 0, 0};
     int period = 6;              // steps after which the launch pattern repeats
     bool corr_in_graph = false;  // correction steps are part of the captured pattern
+    int cluster_ctas = 0;        // small lattice without a squirmer: CTAs of k_cluster_steps (0: not used)
+    ClusterWork cluster{};
     bool wallrows_on_a = false;  // wall rows follow the bulk on stream a (short bulk, squirmer chain)
 
     // host mirrors
@@ -179,6 +182,10 @@ int rows_reserve(bool squirmer, int sms) {
     if (e && *e) r = std::atoi(e);
     return std::max(0, std::min(r, sms / 2));
 }
+
+// Steps per k_cluster_steps launch, at most (a launch of the smallest duct then
+// takes about a fifth of a second).
+constexpr int CLUSTER_MAX_STEPS = 1 << 17;
 
 // Capacity of the boundary-link list of a lattice with these parameters (the
 // links lie inside the sphere's box, so the box volume bounds them).
@@ -769,6 +776,8 @@ int create_impl(const lbmgpu_params* p, const MemberOpts* mo, lbmgpu_handle** ou
             }
         }
     }
+    // LBMGPU_BULK names a kernel of the separate launches
+    if (!h->has_sq && !mo && !std::getenv("LBMGPU_BULK")) h->cluster_ctas = h->lz->cluster_fit(L, h->cluster);
     h->link_cap = link_capacity(*p);
     h->chg_cap = h->link_cap;
     if ((long long)hi.links.size() >= h->link_cap) {
@@ -884,6 +893,15 @@ int lbmgpu_run(lbmgpu_handle* h, int nsteps) {
     if (nsteps == 0) return LBMGPU_OK;
     CUDA_TRY(h, cudaSetDevice(h->p.device));
     cudaStream_t sa = h->stream, sb = h->zs;
+    while (h->cluster_ctas && nsteps > 2) {   // all but the last step
+        ClusterWork w = h->cluster;
+        w.nsteps = std::min(nsteps - 1, CLUSTER_MAX_STEPS);
+        w.parity = (int)(h->t_main & 1);
+        CUDA_TRY(h, h->lz->cluster(h->L, h->f, w, h->cluster_ctas, sa));
+        ++h->launches;
+        h->t_main += w.nsteps;
+        nsteps -= w.nsteps;
+    }
     const int per_step = 1 + (h->geom.nwallrows ? 1 : 0) + (h->geom.bgrid ? 1 : 0) + (h->has_sq ? 1 : 0);
     const int gsteps = h->period * ((MIN_GRAPH + h->period - 1) / h->period);
     fused_begin(h, sa, sb);

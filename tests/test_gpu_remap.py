@@ -8,7 +8,10 @@ wider than it is, one that crosses the periodic boundary, one next to a wall,
 and one of 14 cells (about 5,900 links, some 60 changes a step at its speed).
 Node types must equal the oracle's exactly; the fields and the rigid body agree
 to 1e-10 (both sides do the same FP64 operations but for the order of a few
-sums, 1e-16 each, over at most 120 steps).
+sums, 1e-16 each, over at most 120 steps). The smallest box amplifies that
+order by 1e6 within its 120 steps: the oracle's own runs, whose force sums
+change order with the threads, are up to 2.4e-10 apart in u (300 runs), so no
+two implementations agree to 1e-10 there; it gets four times that.
 """
 import numpy as np
 import pytest
@@ -40,9 +43,10 @@ def test_remap_follows_the_oracle(case, oracle_mod):
     flo, ro, uo = o.fields()
     assert np.array_equal(flag, flo)
     fluid = flo == 0
-    assert np.linalg.norm(u[fluid] - uo[fluid]) <= 1e-10 * np.linalg.norm(uo[fluid])
+    tol = 1e-9 if case == "tiny" else 1e-10
+    assert np.linalg.norm(u[fluid] - uo[fluid]) <= tol * np.linalg.norm(uo[fluid])
     assert np.linalg.norm(rho[fluid] - ro[fluid]) <= 1e-10 * np.linalg.norm(ro[fluid])
     a, b = s.squirmer(), o.squirmer()
     for k in ("X", "e", "U", "W"):
-        assert np.abs(a[k] - b[k]).max() <= 1e-10, k
+        assert np.abs(a[k] - b[k]).max() <= tol, k
     s.close()
