@@ -53,7 +53,11 @@ __global__ void __launch_bounds__(AUX_BLOCK) k_mass_partial(const Lattice L, con
     for (unsigned n = blockIdx.x * blockDim.x + threadIdx.x; n < L.N; n += gridDim.x * blockDim.x) {
         if ((flag[n] & TYPE_MASK) != T_FLUID) continue;
         const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny), z = (int)(n / L.nxy);
-        for (int i = 0; i < Q; ++i) m += Pop<S>::raw(f, logical_slot(L, P, i, n, x, y, z));
+        double v[Q];   // all loads in flight, then the sum in direction order
+#pragma unroll
+        for (int i = 0; i < Q; ++i) v[i] = Pop<S>::raw(f, logical_slot(L, P, i, n, x, y, z));
+#pragma unroll
+        for (int i = 0; i < Q; ++i) m += v[i];
         c += 1.0;
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -73,11 +77,17 @@ __global__ void __launch_bounds__(AUX_BLOCK) k_mass_partial(const Lattice L, con
 // correction still pending from the time loop (applied on the next load) is
 // folded in: it would add w_i*d_p to every population of every fluid node,
 // i.e. nf*d_p to m. The total is applied at once and nothing stays pending.
+// The partials are fetched by the whole CTA and added in order by one thread
+// (38 us when that thread also fetched them, one round trip after another).
 template <class S>
-__global__ void k_mass_final(const double* part, int nparts, SqState* sq, double* dflag) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__global__ void __launch_bounds__(AUX_BLOCK) k_mass_final(const double* part, SqState* sq, double* dflag) {
+    __shared__ double2 sh[MASS_GRID];
+    for (int b = threadIdx.x; b < MASS_GRID; b += AUX_BLOCK) sh[b] = make_double2(part[2 * b], part[2 * b + 1]);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
     double m = 0, c = 0;
-    for (int b = 0; b < nparts; ++b) { m += part[2 * b]; c += part[2 * b + 1]; }
+#pragma unroll 8
+    for (int b = 0; b < MASS_GRID; ++b) { m += sh[b].x; c += sh[b].y; }
     if (c == 0.0) { *dflag = 0.0; return; }
     const double dp = sq->corr_pending ? sq->corr_d : 0.0;
     m += c * dp;
@@ -95,10 +105,11 @@ __global__ void k_mass_apply(const Lattice L, void* f, const uint8_t* flag, int 
     for (unsigned n = blockIdx.x * blockDim.x + threadIdx.x; n < L.N; n += gridDim.x * blockDim.x) {
         if ((flag[n] & TYPE_MASK) != T_FLUID) continue;
         const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny), z = (int)(n / L.nxy);
-        for (int i = 0; i < Q; ++i) {
-            const size_t k = logical_slot(L, P, i, n, x, y, z);
-            Pop<S>::put(f, k, i, Pop<S>::get(f, k, i) + w_rt(i) * d);
-        }
+        double v[Q];
+#pragma unroll
+        for (int i = 0; i < Q; ++i) v[i] = Pop<S>::get(f, logical_slot(L, P, i, n, x, y, z), i);
+#pragma unroll
+        for (int i = 0; i < Q; ++i) Pop<S>::put(f, logical_slot(L, P, i, n, x, y, z), i, v[i] + w_rt(i) * d);
     }
 }
 

@@ -136,7 +136,7 @@ template <class S>
 static void correct_mass_launch(const Lattice& L, void* f, const uint8_t* flag, int P, SqState* sq, double* part,
                                 double* dflag, cudaStream_t st) {
     k_mass_partial<S><<<MASS_GRID, AUX_BLOCK, 0, st>>>(L, f, flag, P, part);
-    k_mass_final<S><<<1, 32, 0, st>>>(part, MASS_GRID, sq, dflag);
+    k_mass_final<S><<<1, AUX_BLOCK, 0, st>>>(part, sq, dflag);
     k_mass_apply<S><<<1184, AUX_BLOCK, 0, st>>>(L, f, flag, P, sq, dflag);
 }
 

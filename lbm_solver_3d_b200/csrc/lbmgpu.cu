@@ -96,6 +96,7 @@ struct lbmgpu_handle {
     SqState* sq = nullptr;
     double* scratch = nullptr;   // N doubles
     double* small = nullptr;     // reduction partials / results
+    int* host_status = nullptr;  // page-locked: the status word after a call
 
     // launch geometry
     StreamGeom geom{};
@@ -491,6 +492,7 @@ void free_all(lbmgpu_handle* h) {
                     h->cand, h->mark, h->traj, h->sq, h->scratch, h->small, h->shell, h->shell_hdr,
                     h->packed, h->snap};
     for (void* q : ptrs) if (q) cudaFree(q);
+    if (h->host_status) cudaFreeHost(h->host_status);
     for (cudaEvent_t e : {h->ev_b[0], h->ev_b[1], h->ev_z, h->ev_s, h->ev_fork, h->ev_join, h->snap_ready})
         if (e) cudaEventDestroy(e);
     for (cudaStream_t s : {h->own, h->zs, h->cap, h->cap2, h->snap_stream})
@@ -607,9 +609,11 @@ void pack_fields(lbmgpu_handle* h, unsigned char* buf, cudaStream_t st) {
 
 int check_status(lbmgpu_handle* h) {
     CUDA_TRY(h, cudaGetLastError());
-    int st = 0;
-    CUDA_TRY(h, cudaMemcpyAsync(&st, &h->sq->status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    int own = 0;   // ensemble members have no page-locked word
+    int* const word = h->host_status ? h->host_status : &own;
+    CUDA_TRY(h, cudaMemcpyAsync(word, &h->sq->status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    const int st = *word;
     if (st & ST_NAN) return fail(h, LBMGPU_ERR_NAN, "non-finite squirmer force, torque or state");
     if (st & ST_REMAP_RANGE)
         return fail(h, LBMGPU_ERR_DEVICE, "squirmer moved one lattice cell or more in a single step");
@@ -701,6 +705,7 @@ int create_impl(const lbmgpu_params* p, const MemberOpts* mo, lbmgpu_handle** ou
         for (cudaEvent_t* e : {&h->ev_b[0], &h->ev_b[1], &h->ev_z, &h->ev_s, &h->ev_fork, &h->ev_join})
             CTRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         h->stream = h->own;
+        CTRY(cudaHostAlloc(reinterpret_cast<void**>(&h->host_status), sizeof(int), cudaHostAllocDefault));
     }
 
     Lattice& L = h->L;
@@ -939,8 +944,9 @@ int lbmgpu_run(lbmgpu_handle* h, int nsteps) {
     return check_status(h);
 }
 
-// LBM::step alone: both collide-stream kernels, then the sphere force of the
-// step (lbm.cpp:219-223), all on the caller's stream.
+// LBM::step alone: the collide-stream kernels, which touch disjoint slots (the
+// wall rows and the zone beside the bulk on the second stream), then the wall
+// force and the sphere force of the step (lbm.cpp:219-223) on the caller's.
 int lbmgpu_step(lbmgpu_handle* h) {
     if (!h) return LBMGPU_ERR_INVALID;
     if (h->member) return fail(h, LBMGPU_ERR_INVALID, "handle belongs to an ensemble: advance it with lbmgpu_batch_run");
@@ -948,16 +954,21 @@ int lbmgpu_step(lbmgpu_handle* h) {
     StepPlan sp = plan_step(h, h->t_main + 1, true, h->pending_corr);
     sp.corr = false;
     const StreamArgs a = stream_args(h, sp);
-    cudaStream_t st = h->stream;
+    cudaStream_t st = h->stream, sb = h->zs;
+    CUDA_TRY(h, cudaEventRecord(h->ev_fork, st));
     h->lz->bulk(sp.par, h->has_sq != 0, true, h->L, a, h->geom, st);
-    if (h->geom.nwallrows) { h->lz->wallrows(sp.par, h->has_sq != 0, true, h->L, a, h->geom, st); ++h->launches; }
-    if (h->geom.bgrid) { h->lz->zone(sp.par, h->has_sq != 0, true, h->L, a, h->geom, st); ++h->launches; }
+    if (h->geom.nwallrows || h->geom.bgrid) {
+        CUDA_TRY(h, cudaStreamWaitEvent(sb, h->ev_fork, 0));
+        if (h->geom.nwallrows) { h->lz->wallrows(sp.par, h->has_sq != 0, true, h->L, a, h->geom, sb); ++h->launches; }
+        if (h->geom.bgrid) { h->lz->zone(sp.par, h->has_sq != 0, true, h->L, a, h->geom, sb); ++h->launches; }
+        fused_end(h, st, sb);
+    }
     k_finalize<<<1, 256, 0, st>>>(h->block_part, h->nblocks, h->block_part_b, h->geom.bgrid ? h->nblocks_b : 0, h->sq);
     h->launches += 2;
     if (h->has_sq) {
+        // the update also marks a pending mass correction as applied
         h->lz->squirmer(h->L, squirmer_args(h, sp.par ^ 1, STAGE_FORCE, 0, -1, -1), st);
-        k_clear_pending<<<1, 32, 0, st>>>(h->sq);
-        h->launches += 2;
+        ++h->launches;
     }
     h->pending_corr = false;
     ++h->t_main;
