@@ -1034,6 +1034,7 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX, RowsCfg<S>::MINB) k_bulk_row
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nx = L.nx, nupd = nx >> 5;
     const size_t stage = rows_stage_bytes<S>(nx);
+    bulk_begin(a.late_wait != 0);
     if (tid == 0) {
         for (int q = 0; q < NST; ++q) {
             mbar_init(&full[q], 1);
@@ -1102,6 +1103,7 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX, RowsCfg<S>::MINB) k_bulk_row
         }
     }
     rows_finish<NST>(w, full, s_abort, s_issued, tid);
+    bulk_end(a.late_wait != 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -1145,6 +1147,7 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX / 2, Rows2Cfg<S>::MINB) k_bul
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nx = L.nx, nupd = nx >> 6;
     const size_t stage = rows_stage_bytes<S>(nx);
+    bulk_begin(a.late_wait != 0);
     if (tid == 0) {
         for (int q = 0; q < NST; ++q) {
             mbar_init(&full[q], 1);
@@ -1248,6 +1251,7 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX / 2, Rows2Cfg<S>::MINB) k_bul
         if (stored) bulk_wait_all();
     }
     rows_finish<NST>(w, full, s_abort, s_issued, tid);
+    bulk_end(a.late_wait != 0);
 }
 
 // One CTA per zone block of every member: zblocks lists the (member, block)

@@ -772,14 +772,17 @@ __global__ void __launch_bounds__(256, bulk_min_blocks<S>(DENSE)) k_bulk(const L
 // multiple of 32. The rows away from walls of one z-plane are one contiguous
 // range of nodes; 256 threads take 256 consecutive nodes of it, so no lane
 // idles at a row's end. Grid (ceil(range / 256), planes away from z walls).
-template <class S, int PAR, bool SQ, bool DENSE = false>
+// LATE: the step's wall rows were launched in front (bulk_begin).
+template <class S, int PAR, bool SQ, bool DENSE = false, bool LATE = false>
 __global__ void __launch_bounds__(256, bulk_min_blocks<S>(DENSE)) k_bulk_flat(const Lattice L, const StreamArgs a) {
-    pdl_wait();
-    pdl_launch_dependents();
+    bulk_begin(LATE);
     const int ylo = L.walls_y ? 2 : 0, rows = L.walls_y ? L.ny - 4 : L.ny;
     const int z = (L.walls_z ? 2 : 0) + (int)blockIdx.y;
     const int o = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (o >= rows * L.nx) return;
+    if (o >= rows * L.nx) {
+        bulk_end(LATE);
+        return;
+    }
     const int dy = o / L.nx;
     const int x = o - dy * L.nx, y = ylo + dy;
     const unsigned n = (unsigned)x + (unsigned)L.nx * ((unsigned)y + (unsigned)L.ny * (unsigned)z);
@@ -787,6 +790,7 @@ __global__ void __launch_bounds__(256, bulk_min_blocks<S>(DENSE)) k_bulk_flat(co
     if (SQ && active) active = !in_zone(L, a.sq->zone[a.zslot], x, y, z);
     NodeSums sums;
     if (active) update_node<S, PAR, false, false>(L, a, n, x, y, z, 0, 0, false, sums);
+    bulk_end(LATE);
 }
 
 // ---------------------------------------------------------------------------

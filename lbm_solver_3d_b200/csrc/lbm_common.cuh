@@ -244,6 +244,7 @@ struct StreamArgs {
     int do_mass;                  // sum the stored populations (a correction step)
     int apply_corr;               // add the pending correction on load (after one)
     int* row_claim;               // staged-row bulk: row counter and CTAs done (RowsWork)
+    int late_wait;                // the bulk follows this step's wall rows and runs beside them (bulk_begin)
 };
 
 // ---- ensembles (k_batch.cuh) -------------------------------------------------
@@ -257,6 +258,20 @@ constexpr int BATCH_MAX_NX = 256;   // longest x-row of an ensemble member
 // no-ops for an ordinary launch.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Start and end of a bulk kernel. Usually it waits for its predecessor, the
+// bulk of the step before. Where the wall rows of the same step are launched
+// in front of it (late), they have themselves waited for that bulk before they
+// let this kernel start, and the two touch disjoint slots: it starts at once
+// and waits for them only before it ends, so that its end still means the end
+// of both.
+__device__ __forceinline__ void bulk_begin(bool late) {
+    if (!late) pdl_wait();
+    pdl_launch_dependents();
+}
+__device__ __forceinline__ void bulk_end(bool late) {
+    if (late) pdl_wait();
+}
 
 struct RowRef {
     int m, y, z;       // member, row coordinates

@@ -25,46 +25,12 @@ static size_t rows2_smem(int nx) {
     else return 0;
 }
 
-template <class S, int PAR, bool SQ, bool MACRO>
-static void bulk_one(const Lattice& L, const StreamArgs& a, const StreamGeom& g, cudaStream_t st) {
-    if (g.rows_grid) {   // rows staged in shared memory (every step; sums in k_bulk's order)
-        const RowsWork w{g.rows_nry, g.rows_n, g.rows_ylo, g.rows_zlo, g.rows_reserve, a.row_claim};
-        if constexpr (S::shifted && !MACRO) {
-            if (g.rows_pairs && !a.do_mass) {   // no sums this step: two nodes per update thread
-                k_bulk_rows2<S, PAR, SQ><<<g.rows_grid, 32 + L.nx / 2, rows2_smem<S>(L.nx), st>>>(L, a, w);
-                return;
-            }
-        }
-        if (MACRO || a.do_mass)
-            k_bulk_rows<S, PAR, SQ, MACRO, true><<<g.rows_grid, 32 + L.nx, rows_smem<S>(L.nx), st>>>(L, a, w);
-        else
-            k_bulk_rows<S, PAR, SQ, false, false><<<g.rows_grid, 32 + L.nx, rows_smem<S>(L.nx), st>>>(L, a, w);
-        return;
-    }
-    if constexpr (S::shifted && !MACRO) {
-        if (!a.do_mass && g.pair.x) {   // no sums this step: two x-adjacent nodes per thread
-            if (L.force_free) k_bulk_pair<S, PAR, SQ, false><<<g.pair, g.pair_block, 0, st>>>(L, a);
-            else k_bulk_pair<S, PAR, SQ, true><<<g.pair, g.pair_block, 0, st>>>(L, a);
-            return;
-        }
-    }
-    if (!MACRO && !a.do_mass && g.flat.x) {   // no sums this step: whole rows of nodes per block
-        if (!S::shifted && g.dense) k_bulk_flat<S, PAR, SQ, true><<<g.flat, 256, 0, st>>>(L, a);
-        else k_bulk_flat<S, PAR, SQ><<<g.flat, 256, 0, st>>>(L, a);
-        return;
-    }
-    if constexpr (!S::shifted) {
-        if (g.dense) {
-            k_bulk<S, PAR, SQ, MACRO, false, true><<<g.grid, g.block, 0, st>>>(L, a);
-            return;
-        }
-    }
-    k_bulk<S, PAR, SQ, MACRO, false><<<g.grid, g.block, 0, st>>>(L, a);
-}
 // Launch with programmatic stream serialisation: the kernel may be scheduled
 // while its predecessor in the stream finishes, and waits for it in pdl_wait().
-// Used on the stream of the chain wall rows -> zone -> squirmer update, whose
-// kernels follow one another step after step.
+// Used on the stream of the chain wall rows -> zone -> squirmer update and on
+// that of the staged-row bulks, whose kernels follow one another step after
+// step (a bulk launched in the ordinary way started about 4 us after the one
+// before ended; a grid of several waves gains nothing from it).
 template <class... KArgs, class... Args>
 static void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
@@ -80,6 +46,43 @@ static void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
     cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+template <class S, int PAR, bool SQ, bool MACRO>
+static void bulk_one(const Lattice& L, const StreamArgs& a, const StreamGeom& g, cudaStream_t st) {
+    if (g.rows_grid) {   // rows staged in shared memory (every step; sums in k_bulk's order)
+        const RowsWork w{g.rows_nry, g.rows_n, g.rows_ylo, g.rows_zlo, g.rows_reserve, a.row_claim};
+        if constexpr (S::shifted && !MACRO) {
+            if (g.rows_pairs && !a.do_mass) {   // no sums this step: two nodes per update thread
+                launch_pdl(k_bulk_rows2<S, PAR, SQ>, dim3(g.rows_grid), dim3(32 + L.nx / 2), rows2_smem<S>(L.nx), st, L, a, w);
+                return;
+            }
+        }
+        if (MACRO || a.do_mass)
+            launch_pdl(k_bulk_rows<S, PAR, SQ, MACRO, true>, dim3(g.rows_grid), dim3(32 + L.nx), rows_smem<S>(L.nx), st, L, a, w);
+        else
+            launch_pdl(k_bulk_rows<S, PAR, SQ, false, false>, dim3(g.rows_grid), dim3(32 + L.nx), rows_smem<S>(L.nx), st, L, a, w);
+        return;
+    }
+    if constexpr (S::shifted && !MACRO) {
+        if (!a.do_mass && g.pair.x) {   // no sums this step: two x-adjacent nodes per thread
+            if (L.force_free) k_bulk_pair<S, PAR, SQ, false><<<g.pair, g.pair_block, 0, st>>>(L, a);
+            else k_bulk_pair<S, PAR, SQ, true><<<g.pair, g.pair_block, 0, st>>>(L, a);
+            return;
+        }
+    }
+    if (!MACRO && !a.do_mass && g.flat.x) {   // no sums this step: whole rows of nodes per block
+        if (a.late_wait) launch_pdl(k_bulk_flat<S, PAR, SQ, false, true>, g.flat, dim3(256), 0, st, L, a);
+        else if (!S::shifted && g.dense) k_bulk_flat<S, PAR, SQ, true><<<g.flat, 256, 0, st>>>(L, a);
+        else k_bulk_flat<S, PAR, SQ><<<g.flat, 256, 0, st>>>(L, a);
+        return;
+    }
+    if constexpr (!S::shifted) {
+        if (g.dense) {
+            k_bulk<S, PAR, SQ, MACRO, false, true><<<g.grid, g.block, 0, st>>>(L, a);
+            return;
+        }
+    }
+    k_bulk<S, PAR, SQ, MACRO, false><<<g.grid, g.block, 0, st>>>(L, a);
+}
 template <class S, int PAR, bool SQ, bool MACRO>
 static void wallrows_one(const Lattice& L, const StreamArgs& a, const StreamGeom& g, cudaStream_t st) {
     if (g.nwallrows) launch_pdl(k_bulk<S, PAR, SQ, MACRO, true>, dim3(g.grid.x, g.nwallrows, 1), g.block, 0, st, L, a);

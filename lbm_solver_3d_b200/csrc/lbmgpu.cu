@@ -105,7 +105,8 @@ struct lbmgpu_handle {
     bool corr_in_graph = false;  // correction steps are part of the captured pattern
     int cluster_ctas = 0;        // small lattice without a squirmer: CTAs of k_cluster_steps (0: not used)
     ClusterWork cluster{};
-    bool wallrows_on_a = false;  // wall rows follow the bulk on stream a (short bulk, squirmer chain)
+    bool wallrows_on_a = false;  // wall rows on stream a with the bulk (short bulk, squirmer chain)
+    bool short_bulk = false;     // shorter still: see create_impl
 
     // host mirrors
     long long t_main = 0;        // time steps issued (AA parity; step s = t_main + 1)
@@ -220,6 +221,7 @@ StreamArgs stream_args(lbmgpu_handle* h, const StepPlan& sp) {
     a.sq = h->sq;
     a.zslot = sp.zslot; a.do_mass = sp.corr ? 1 : 0; a.apply_corr = sp.apply ? 1 : 0;
     a.row_claim = h->row_claim;
+    a.late_wait = 0;
     return a;
 }
 
@@ -515,13 +517,19 @@ StepPlan plan_step(lbmgpu_handle* h, long long s, bool macro, bool apply) {
 // marks B(s-1)... precisely: ev_b[(s-1)&1] marks B(s-1), ev_z marks Z(s-1) and
 // ev_s marks S(s-1).
 void issue_fused(lbmgpu_handle* h, cudaStream_t sa, cudaStream_t sb, const StepPlan& sp) {
-    const StreamArgs a = stream_args(h, sp);
+    StreamArgs a = stream_args(h, sp);
     const int par = sp.par;
     cudaStreamWaitEvent(sa, h->ev_z, 0);
     if (sp.apply) cudaStreamWaitEvent(sa, h->ev_s, 0);
-    h->lz->bulk(par, h->has_sq != 0, sp.macro, h->L, a, h->geom, sa);
     int k = 1;
-    if (h->geom.nwallrows && h->wallrows_on_a) { h->lz->wallrows(par, h->has_sq != 0, sp.macro, h->L, a, h->geom, sa); ++k; }
+    // wall rows on stream a: in front of the bulk, which runs beside them, where
+    // its kernel can (the staged rows; of the others the flat one, if short)
+    const bool on_a = h->geom.nwallrows && h->wallrows_on_a, sums = sp.macro || sp.corr;
+    a.late_wait = on_a && (h->geom.rows_grid || (h->geom.flat.x && !sums && h->short_bulk));
+    if (a.late_wait) h->lz->wallrows(par, h->has_sq != 0, sp.macro, h->L, a, h->geom, sa);
+    h->lz->bulk(par, h->has_sq != 0, sp.macro, h->L, a, h->geom, sa);
+    if (on_a && !a.late_wait) h->lz->wallrows(par, h->has_sq != 0, sp.macro, h->L, a, h->geom, sa);
+    k += on_a;
     cudaEventRecord(h->ev_b[sp.s & 1], sa);
     cudaStreamWaitEvent(sb, h->ev_b[(sp.s - 1) & 1], 0);
     if (h->geom.nwallrows && !h->wallrows_on_a) { h->lz->wallrows(par, h->has_sq != 0, sp.macro, h->L, a, h->geom, sb); ++k; }
@@ -739,8 +747,13 @@ int create_impl(const lbmgpu_params* p, const MemberOpts* mo, lbmgpu_handle** ou
     // the bulk of the same step needs, so they may go on either stream. On
     // stream b they overlap the bulk but lengthen the chain wall rows -> zone ->
     // squirmer; when the bulk moves less than ~200 MB (about 40 us) that chain
-    // is the step, and they go after the bulk on stream a instead.
+    // is the step, and they go on stream a instead, in front of a bulk that runs
+    // beside them (issue_fused). For the flat kernel that pays only while the
+    // bulk is short: 70x50x60 FP32 (32 MB) 20.7 -> 19.1 us a step, 100x90x70
+    // FP16 (48 MB) 27.8 -> 27.1, but 149x97x83 FP16 (91 MB) 40.8 -> 42.3 and
+    // FP32 (182 MB) 61.7 -> 62.5.
     h->wallrows_on_a = h->has_sq && (double)Q * 2.0 * h->esize * (double)N <= 200e6;
+    h->short_bulk = (double)Q * 2.0 * h->esize * (double)N <= 64e6;
     // FP64: a long bulk runs denser (3 CTAs/SM); a short one keeps 2, which
     // leaves room on the SMs for the zone and squirmer chain beside it
     h->geom.dense = (double)Q * 2.0 * h->esize * (double)N > 200e6;
