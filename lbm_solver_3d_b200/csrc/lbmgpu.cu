@@ -173,14 +173,29 @@ int bulk_kind() {
     return 0;
 }
 
-// SMs the persistent staged-row bulk leaves to the squirmer update of the
-// second stream, whose CTA needs an SM to itself (a zone CTA fits beside the
-// bulk's CTAs on any SM): LBMGPU_ROWS_RESERVE, else ROWS_RESERVE with a
-// squirmer and none without one.
-constexpr int ROWS_RESERVE = 2;
-int rows_reserve(bool squirmer, int sms) {
+// SMs the persistent staged-row bulk leaves to the zone and squirmer kernels of
+// the second stream: LBMGPU_ROWS_RESERVE, else by this rule with a squirmer and
+// none without one.
+//   2  the squirmer update's CTA needs an SM to itself; a zone CTA (64 threads
+//      of 128 registers) fits beside at most 18 of the bulk's warps on any SM.
+//   8  for a bulk of 200 MB or more, where the second stream has more to do
+//      than that: its wall rows too, or (FP32 and FP64) more bulk warps are
+//      resident (nx = 128: 20). Its kernels then started as the bulk's CTAs
+//      retired, and the next bulk waited for them. Steps with 2 -> 8: walls,
+//      192x96x96 FP32 74.6 -> 69.8 us, FP64 99.2 -> 94.2, 256x128x128 FP32
+//      132.1 -> 126.7, FP64 210.1 -> 201.8, FP16 99.0 -> 92.2; 128x128x128
+//      without walls FP32 72.7 -> 67.9, FP64 111.9 -> 104.4. Shorter bulks
+//      feel the lost SMs more: 128x96x96 FP32 (179 MB) 42.2 -> 44.5. In the
+//      other cases gains and losses balance: 256x128x128 FP32 125.8 -> 128.0,
+//      FP64 201.9 -> 204.3.
+//   4  the FP16 two-node kernel (20 warps) from 170 MB: 256x128x128 96.4 ->
+//      92.0, 256x96x96 60.7 -> 57.0; 192x96x96 (134 MB) 50.2 -> 51.3.
+int rows_reserve(bool squirmer, bool walls, int sms, bool pairs, int warps_per_sm, double bytes) {
     const char* e = std::getenv("LBMGPU_ROWS_RESERVE");
-    int r = squirmer ? ROWS_RESERVE : 0;
+    int r = 2;
+    if (bytes >= 200e6 && (walls || (!pairs && warps_per_sm > 18))) r = 8;
+    else if (pairs && bytes >= 170e6) r = 4;
+    if (!squirmer) r = 0;
     if (e && *e) r = std::atoi(e);
     return std::max(0, std::min(r, sms / 2));
 }
@@ -790,7 +805,10 @@ int create_impl(const lbmgpu_params* p, const MemberOpts* mo, lbmgpu_handle** ou
                 h->geom.rows_ylo = p->walls_y ? 2 : 0;
                 h->geom.rows_zlo = p->walls_z ? 2 : 0;
                 h->geom.rows_grid = (unsigned)std::min<long long>((long long)sms * per_sm, (long long)rows * planes);
-                h->geom.rows_reserve = rows_reserve(h->has_sq != 0, sms);
+                const bool pairs = h->geom.rows_pairs;
+                h->geom.rows_reserve = rows_reserve(h->has_sq != 0, h->geom.nwallrows > 0, sms, pairs,
+                                                    per_sm * (1 + p->nx / (pairs ? 64 : 32)),
+                                                    (double)Q * 2.0 * h->esize * (double)N);
             }
         }
     }
