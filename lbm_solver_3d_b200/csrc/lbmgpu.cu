@@ -96,7 +96,7 @@ struct lbmgpu_handle {
     SqState* sq = nullptr;
     double* scratch = nullptr;   // N doubles
     double* small = nullptr;     // reduction partials / results
-    int* host_status = nullptr;  // page-locked: the status word after a call
+    int* host_status = nullptr;  // page-locked: the status word after a call (status_word; null: not yet)
 
     // launch geometry
     StreamGeom geom{};
@@ -630,9 +630,23 @@ void pack_fields(lbmgpu_handle* h, unsigned char* buf, cudaStream_t st) {
     ++h->launches;
 }
 
+// A page-locked status word for a program that steps call by call, where each
+// call reads the status. Allocating it takes 1 to 2 ms, more than its few us a
+// call are worth to one that creates a lattice and calls lbmgpu_run on it.
+void status_word(lbmgpu_handle* h) {
+    if (h->host_status) return;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // another thread may be capturing
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaHostAlloc(reinterpret_cast<void**>(&h->host_status), sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        h->host_status = nullptr;   // pageable, as for lbmgpu_run
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+}
+
 int check_status(lbmgpu_handle* h) {
     CUDA_TRY(h, cudaGetLastError());
-    int own = 0;   // ensemble members have no page-locked word
+    int own = 0;
     int* const word = h->host_status ? h->host_status : &own;
     CUDA_TRY(h, cudaMemcpyAsync(word, &h->sq->status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -728,7 +742,6 @@ int create_impl(const lbmgpu_params* p, const MemberOpts* mo, lbmgpu_handle** ou
         for (cudaEvent_t* e : {&h->ev_b[0], &h->ev_b[1], &h->ev_z, &h->ev_s, &h->ev_fork, &h->ev_join})
             CTRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         h->stream = h->own;
-        CTRY(cudaHostAlloc(reinterpret_cast<void**>(&h->host_status), sizeof(int), cudaHostAllocDefault));
     }
 
     Lattice& L = h->L;
@@ -982,6 +995,7 @@ int lbmgpu_step(lbmgpu_handle* h) {
     if (!h) return LBMGPU_ERR_INVALID;
     if (h->member) return fail(h, LBMGPU_ERR_INVALID, "handle belongs to an ensemble: advance it with lbmgpu_batch_run");
     CUDA_TRY(h, cudaSetDevice(h->p.device));
+    status_word(h);
     StepPlan sp = plan_step(h, h->t_main + 1, true, h->pending_corr);
     sp.corr = false;
     const StreamArgs a = stream_args(h, sp);
