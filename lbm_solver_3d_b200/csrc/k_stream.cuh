@@ -226,6 +226,21 @@ struct GlobalSrc {
     }
 };
 
+// Populations already in registers: a node's are loaded together with its type,
+// so that one memory latency covers both; one that turns out not to be updated
+// has loaded them for nothing.
+template <class S>
+using HeldPop = std::conditional_t<S::shifted, float, double>;
+template <class V>
+struct HeldSrc {
+    const V* held;
+    template <class S, int PAR, class W>
+    __device__ __forceinline__ void load(const typename S::T*, unsigned, unsigned, const Nbr&, W* v) const {
+#pragma unroll
+        for (int i = 0; i < Q; ++i) v[i] = held[i];
+    }
+};
+
 // a / b, correctly rounded, given y = 1 / b correctly rounded (Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor",
 // 1990): the residual of a y is exact in one FMA and the corrected quotient
@@ -744,8 +759,15 @@ __host__ __device__ constexpr int bulk_min_blocks(bool dense) {
 //  squirmer update writes (except the correction value on the step after a
 //  correction step, when the launch waits for it).
 // ---------------------------------------------------------------------------
-//    DENSE (FP64 only) 3 CTAs/SM instead of 2 (80 registers, a few spills): for
-//          long bulks; a short one leaves room for the zone and squirmer chain
+//    DENSE (FP64 only) 3 CTAs/SM instead of 2 (80 registers, some spills): for
+//          long bulks; a short one leaves room for the zone and squirmer chain.
+//          The populations are loaded beside the type instead of after it
+//          (HeldSrc), although that spills 112 bytes: with 24 warps per SM the
+//          kernel is bound by those two latencies. Steps: 201x130x117 198.5 ->
+//          178.4 us (0.72 -> 0.80 of the copy rate), 300x100x100 slit 194.1 ->
+//          177.2, 384x96x96 216.5 -> 202.5, 149x97x83 slit 87.9 -> 82.7. The
+//          shifted forms and the ensemble's chunks gained nothing from it (FP32
+//          201x130x117 137.5 -> 140.3, FP16 384x96x96 99.3 -> 103.1).
 template <class S, int PAR, bool SQ, bool MACRO, bool WR, bool DENSE = false>
 __global__ void __launch_bounds__(256, bulk_min_blocks<S>(DENSE)) k_bulk(const Lattice L, const StreamArgs a) {
     pdl_wait();
@@ -758,10 +780,18 @@ __global__ void __launch_bounds__(256, bulk_min_blocks<S>(DENSE)) k_bulk(const L
     if (!WR && wr) return;  // block-uniform: the wall-row launch owns this row and its partials
     const unsigned n = (unsigned)x + (unsigned)L.nx * ((unsigned)y + (unsigned)L.ny * (unsigned)z);
     // FLUID with no PARTICLE neighbour; wall neighbours are whole layers
-    bool active = x < L.nx && (a.flag[n] & (uint8_t)~NEAR_WALL) == 0;
+    bool active = x < L.nx;
+    HeldPop<S> held[DENSE ? Q : 1];
+    if (DENSE && active) load_node<S, PAR>(static_cast<const typename S::T*>(a.f), L.N, n, Nbr(L, x, y, z), held);
+    active = active && (a.flag[n] & (uint8_t)~NEAR_WALL) == 0;
     if (SQ && active) active = !in_zone(L, a.sq->zone[a.zslot], x, y, z);
     NodeSums sums;
-    if (active) update_node<S, PAR, false, MACRO>(L, a, n, x, y, z, 0, WR ? wr : (uint8_t)0, MACRO, sums);
+    if (active) {
+        if constexpr (DENSE)
+            update_node<S, PAR, false, MACRO>(L, a, n, x, y, z, 0, WR ? wr : (uint8_t)0, MACRO, sums, HeldSrc<HeldPop<S>>{held});
+        else
+            update_node<S, PAR, false, MACRO>(L, a, n, x, y, z, 0, WR ? wr : (uint8_t)0, MACRO, sums);
+    }
     if (a.do_mass || MACRO) {
         const unsigned bid = blockIdx.x + gridDim.x * ((unsigned)y + (unsigned)L.ny * (unsigned)z);
         block_reduce4<256>(sums.fw[0], sums.fw[1], sums.fw[2], sums.mass, a.block_part + (size_t)bid * BLOCK_PART);
@@ -787,10 +817,15 @@ __global__ void __launch_bounds__(256, bulk_min_blocks<S>(DENSE)) k_bulk_flat(co
     const int dy = o / L.nx;
     const int x = o - dy * L.nx, y = ylo + dy;
     const unsigned n = (unsigned)x + (unsigned)L.nx * ((unsigned)y + (unsigned)L.ny * (unsigned)z);
+    HeldPop<S> held[DENSE ? Q : 1];
+    if (DENSE) load_node<S, PAR>(static_cast<const typename S::T*>(a.f), L.N, n, Nbr(L, x, y, z), held);
     bool active = (a.flag[n] & (uint8_t)~NEAR_WALL) == 0;
     if (SQ && active) active = !in_zone(L, a.sq->zone[a.zslot], x, y, z);
     NodeSums sums;
-    if (active) update_node<S, PAR, false, false>(L, a, n, x, y, z, 0, 0, false, sums);
+    if (active) {
+        if constexpr (DENSE) update_node<S, PAR, false, false>(L, a, n, x, y, z, 0, 0, false, sums, HeldSrc<HeldPop<S>>{held});
+        else update_node<S, PAR, false, false>(L, a, n, x, y, z, 0, 0, false, sums);
+    }
     bulk_end(LATE);
 }
 
@@ -1127,18 +1162,6 @@ __device__ __forceinline__ void zone_particle_links(const Lattice& L, const Stre
     }
 }
 
-// Populations already in registers (zone_cell loads them before it knows the
-// node's type).
-template <class V>
-struct HeldSrc {
-    const V* held;
-    template <class S, int PAR, class W>
-    __device__ __forceinline__ void load(const typename S::T*, unsigned, unsigned, const Nbr&, W* v) const {
-#pragma unroll
-        for (int i = 0; i < Q; ++i) v[i] = held[i];
-    }
-};
-
 // Cell k of the zone whose corner is (lx, ly, lz), one per thread (every lane
 // of the warp calls it; sync() runs before the particle links read sq);
 // returns the sums for the block reduction. sq is the block's copy of the
@@ -1152,7 +1175,7 @@ __device__ __forceinline__ void zone_cell(const Lattice& L, const StreamArgs& a,
     unsigned n = 0;
     int x = 0, y = 0, z = 0;
     uint8_t fl = T_WALL;
-    using V = std::conditional_t<S::shifted, float, double>;
+    using V = HeldPop<S>;
     V held[Q];
     if (SQ && k < a.zone_cells) {
         const int bx = k % a.zw[0], by = (k / a.zw[0]) % a.zw[1], bz = k / (a.zw[0] * a.zw[1]);
