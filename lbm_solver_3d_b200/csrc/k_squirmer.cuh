@@ -374,6 +374,7 @@ __device__ __forceinline__ void remap_few(const Lattice& L, const SqArgs& a, SqS
             w.part[e][4] = sg * (r[2] * p[0] - r[0] * p[2]);
             w.part[e][5] = sg * (r[0] * p[1] - r[1] * p[0]);
         }
+        __syncwarp();   // part and mass are read by other lanes; a vote does not order memory
         const unsigned unc = __ballot_sync(0xffffffffu, kind == 2);
         if (tid < 6) {   // Fc, Tc: the changes in order
             double* acc = tid < 3 ? &s.Fc[tid] : &s.Tc[tid - 3];
