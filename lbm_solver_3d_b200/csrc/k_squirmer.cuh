@@ -1039,17 +1039,17 @@ __device__ __forceinline__ bool squirmer_update(const Lattice& L, const SqArgs& 
     BodyPre bp;
     if (warp < 2) bp = body_pre(L, s, shell_X, warp, axis);
     if (early && !wait()) return false;
-    if (s.status & (ST_NAN | ST_REMAP_RANGE | ST_LINK_OVERFLOW)) return true;  // invalid already; the host reports it
+    // invalid already; the host reports it. Every warp reads the status before
+    // the next barrier, behind which the body may set bits: one verdict for all.
+    if (s.status & (ST_NAN | ST_REMAP_RANGE | ST_LINK_OVERFLOW)) return true;
 
     const bool loop = (a.stages & STAGE_LOOP) != 0;
     const bool corr_step = loop && a.corr_step;
 
     // ---------------- stages FORCE, BODY ----------------
     const bool force = (a.stages & STAGE_FORCE) != 0, body = (a.stages & STAGE_BODY) != 0;
-    if (force) {
-        link_warp_sums(a.link_part, s.n_links, (size_t)a.link_cap, sh.red);
-        __syncthreads();
-    }
+    if (force) link_warp_sums(a.link_part, s.n_links, (size_t)a.link_cap, sh.red);
+    __syncthreads();
     if (warp == 0) {
         const double F = force ? link_total(sh.red, axis) : s.Fh[axis];
         if (force && lane < 3) s.Fh[lane] = F;
