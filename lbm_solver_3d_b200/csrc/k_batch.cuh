@@ -952,6 +952,8 @@ template <class S, int PAR, int NST>
 __device__ __forceinline__ void rows_produce(const Lattice& L, const StreamArgs& a, const RowsWork& w,
                                              unsigned char* raw, size_t stage, uint64_t* full, uint64_t* empty,
                                              int* rowid, volatile int& s_abort, int& s_issued, int lane) {
+    // what bulk_begin was shown, for the copy engine's reads too
+    if (a.late_wait) asm volatile("fence.proxy.async.global;" ::: "memory");
     for (int k = 0;; ++k) {
         const int q = k % NST;
         int r = 0;
@@ -1034,7 +1036,7 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX, RowsCfg<S>::MINB) k_bulk_row
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nx = L.nx, nupd = nx >> 5;
     const size_t stage = rows_stage_bytes<S>(nx);
-    bulk_begin(a.late_wait != 0);
+    bulk_begin(a, a.late_wait != 0);
     if (tid == 0) {
         for (int q = 0; q < NST; ++q) {
             mbar_init(&full[q], 1);
@@ -1147,7 +1149,7 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX / 2, Rows2Cfg<S>::MINB) k_bul
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nx = L.nx, nupd = nx >> 6;
     const size_t stage = rows_stage_bytes<S>(nx);
-    bulk_begin(a.late_wait != 0);
+    bulk_begin(a, a.late_wait != 0);
     if (tid == 0) {
         for (int q = 0; q < NST; ++q) {
             mbar_init(&full[q], 1);

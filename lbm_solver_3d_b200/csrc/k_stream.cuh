@@ -771,6 +771,7 @@ __host__ __device__ constexpr int bulk_min_blocks(bool dense) {
 template <class S, int PAR, bool SQ, bool MACRO, bool WR, bool DENSE = false>
 __global__ void __launch_bounds__(256, bulk_min_blocks<S>(DENSE)) k_bulk(const Lattice L, const StreamArgs a) {
     pdl_wait();
+    if (WR && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) order_publish(a.order, a.order_tag);
     pdl_launch_dependents();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     int y, z;
@@ -806,7 +807,7 @@ __global__ void __launch_bounds__(256, bulk_min_blocks<S>(DENSE)) k_bulk(const L
 // LATE: the step's wall rows were launched in front (bulk_begin).
 template <class S, int PAR, bool SQ, bool DENSE = false, bool LATE = false>
 __global__ void __launch_bounds__(256, bulk_min_blocks<S>(DENSE)) k_bulk_flat(const Lattice L, const StreamArgs a) {
-    bulk_begin(LATE);
+    bulk_begin(a, LATE);
     const int ylo = L.walls_y ? 2 : 0, rows = L.walls_y ? L.ny - 4 : L.ny;
     const int z = (L.walls_z ? 2 : 0) + (int)blockIdx.y;
     const int o = (int)(blockIdx.x * blockDim.x + threadIdx.x);

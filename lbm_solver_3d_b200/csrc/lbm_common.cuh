@@ -245,6 +245,8 @@ struct StreamArgs {
     int apply_corr;               // add the pending correction on load (after one)
     int* row_claim;               // staged-row bulk: row counter and CTAs done (RowsWork)
     int late_wait;                // the bulk follows this step's wall rows and runs beside them (bulk_begin)
+    int* order;                   // word that the wall rows publish for such a bulk (order_publish), and
+    int order_tag;                // this step's value of it: differs from the two steps' before and after
 };
 
 // ---- ensembles (k_batch.cuh) -------------------------------------------------
@@ -259,14 +261,35 @@ constexpr int BATCH_MAX_NX = 256;   // longest x-row of an ensemble member
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// What a kernel that waits for its predecessor is shown, a kernel behind it that
+// has not waited yet is not: pdl_wait makes earlier writes visible to the grid
+// that calls it. A thread behind its own pdl_wait therefore publishes this
+// step's tag (release), and a thread of the later kernel that reads that tag
+// (acquire) sees all that was visible there. One that does not find it waits
+// itself, so neither ever spins.
+__device__ __forceinline__ void order_publish(int* word, int tag) {
+    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(word), "r"(tag) : "memory");
+}
+__device__ __forceinline__ void order_acquire(const int* word, int tag) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+    if (v != tag) pdl_wait();
+}
+
 // Start and end of a bulk kernel. Usually it waits for its predecessor, the
 // bulk of the step before. Where the wall rows of the same step are launched
 // in front of it (late), they have themselves waited for that bulk before they
-// let this kernel start, and the two touch disjoint slots: it starts at once
-// and waits for them only before it ends, so that its end still means the end
-// of both.
-__device__ __forceinline__ void bulk_begin(bool late) {
-    if (!late) pdl_wait();
+// let this kernel start, and the two touch disjoint slots: it starts at once,
+// with the wall rows' word for what came before them, and waits for them only
+// before it ends, so that its end still means the end of both. Every thread of
+// the CTA calls both.
+__device__ __forceinline__ void bulk_begin(const StreamArgs& a, bool late) {
+    if (late) {
+        if (threadIdx.x == 0) order_acquire(a.order, a.order_tag);
+        __syncthreads();
+    } else {
+        pdl_wait();
+    }
     pdl_launch_dependents();
 }
 __device__ __forceinline__ void bulk_end(bool late) {

@@ -83,7 +83,7 @@ struct lbmgpu_handle {
     unsigned nblocks = 0;
     double* block_part_b = nullptr;
     unsigned nblocks_b = 0;
-    int* row_claim = nullptr;      // staged-row bulk: row counter, CTAs done
+    int* row_claim = nullptr;      // staged-row bulk: row counter, CTAs done; then the order words (order_publish)
     int* ordermap = nullptr;
     int* chg_node = nullptr;
     int* chg_key = nullptr;
@@ -225,6 +225,12 @@ bool is_corr_step(const lbmgpu_handle* h, long long s) {
     return h->has_sq && k > 0 && s % k == 0;
 }
 
+// Words behind row_claim that one kernel of a step publishes for the next, and
+// the step's value: a function of what a captured step keeps, different from
+// that of the steps around it. Zero after a load, whose steps may repeat one.
+constexpr int ORDER_WALL = 2, ROW_WORDS = 3;
+int order_tag(const StepPlan& sp) { return 1 + 2 * sp.zslot + sp.par; }
+
 StreamArgs stream_args(lbmgpu_handle* h, const StepPlan& sp) {
     StreamArgs a;
     a.f = h->f; a.flag = h->flag; a.rho = h->rho; a.ux = h->ux; a.uy = h->uy; a.uz = h->uz;
@@ -237,6 +243,8 @@ StreamArgs stream_args(lbmgpu_handle* h, const StepPlan& sp) {
     a.zslot = sp.zslot; a.do_mass = sp.corr ? 1 : 0; a.apply_corr = sp.apply ? 1 : 0;
     a.row_claim = h->row_claim;
     a.late_wait = 0;
+    a.order = h->row_claim + ORDER_WALL;
+    a.order_tag = order_tag(sp);
     return a;
 }
 
@@ -868,7 +876,7 @@ int create_impl(const lbmgpu_params* p, const MemberOpts* mo, lbmgpu_handle** ou
     CTRY(cudaMalloc(&h->scratch, N * sizeof(double)));
     CTRY(cudaMalloc(&h->block_part, (size_t)h->nblocks * BLOCK_PART * sizeof(double)));
     CTRY(cudaMalloc(&h->block_part_b, (size_t)h->nblocks_b * BLOCK_PART * sizeof(double)));
-    CTRY(cudaMalloc(&h->row_claim, 2 * sizeof(int)));
+    CTRY(cudaMalloc(&h->row_claim, ROW_WORDS * sizeof(int)));
     CTRY(cudaMalloc(&h->wallrows, std::max<size_t>(2, hi.wallrows.size()) * sizeof(int)));
     CTRY(cudaMalloc(&h->sq, sizeof(SqState)));
     CTRY(cudaMalloc(&h->small, (2 * MASS_GRID + 4 * DIAG_GRID + 16) * sizeof(double)));
@@ -894,7 +902,7 @@ int create_impl(const lbmgpu_params* p, const MemberOpts* mo, lbmgpu_handle** ou
     h->launches += 5;
     CTRY(cudaMemsetAsync(h->block_part, 0, (size_t)h->nblocks * BLOCK_PART * sizeof(double), st));
     CTRY(cudaMemsetAsync(h->block_part_b, 0, (size_t)h->nblocks_b * BLOCK_PART * sizeof(double), st));
-    CTRY(cudaMemsetAsync(h->row_claim, 0, 2 * sizeof(int), st));
+    CTRY(cudaMemsetAsync(h->row_claim, 0, ROW_WORDS * sizeof(int), st));
     if (!hi.wallrows.empty())
         CTRY(cudaMemcpyAsync(h->wallrows, hi.wallrows.data(), hi.wallrows.size() * sizeof(int),
                              cudaMemcpyHostToDevice, st));
@@ -1424,6 +1432,7 @@ int lbmgpu_checkpoint_load(lbmgpu_handle* h, const void* buf, size_t len) {
         // which candidates are tested)
         CUDA_TRY(h, cudaMemsetAsync(h->shell_hdr, 0, sizeof(ShellCache), st));
     }
+    CUDA_TRY(h, cudaMemsetAsync(h->row_claim + ORDER_WALL, 0, (ROW_WORDS - ORDER_WALL) * sizeof(int), st));
     CUDA_TRY(h, cudaStreamSynchronize(st));
     CUDA_TRY(h, cudaGetLastError());
     h->t_main = hd.t_main;
