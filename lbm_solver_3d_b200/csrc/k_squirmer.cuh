@@ -46,9 +46,9 @@ constexpr int SQ_PRE = 8;           // candidates per thread fetched ahead: 4096
 constexpr int SQ_FEW = 32;          // changed nodes that remap_few orders: one warp
 constexpr int SQ_FEW_LINKS = 4096;  // boundary links that remap_few edits in shared memory (R up to about 12)
 constexpr int STAGE_BODY = 1, STAGE_REMAP = 2, STAGE_LOOP = 4, STAGE_FORCE = 8;
-// The launch directly follows a zone kernel that had itself waited for the
-// update before: this update may read what that one wrote (its state, the
-// candidate list, the node types) before its own pdl_wait.
+// The launch follows a zone kernel that had itself waited for the update before
+// and published order_tag: this update may read what that one wrote (its state,
+// the candidate list, the node types) before its own pdl_wait.
 constexpr int STAGE_PRE = 16;
 
 struct SqArgs {
@@ -79,6 +79,8 @@ struct SqArgs {
     int stages;
     int corr_step;            // this step is a mass-correction step (time-loop mode)
     int zslot_a, zslot_b;     // zone slots to (re)write from the new position, -1: none
+    const int* order;         // STAGE_PRE: the word that the step's zone kernel publishes, and its value
+    int order_tag;
 };
 
 struct ChgSh {
@@ -1159,7 +1161,9 @@ __device__ __forceinline__ bool squirmer_update(const Lattice& L, const SqArgs& 
 template <class S>
 __global__ void __launch_bounds__(SQ_THREADS, 1) k_squirmer(const __grid_constant__ Lattice L,
                                                          const __grid_constant__ SqArgs a) {
-    squirmer_update<S>(L, a, (a.stages & STAGE_PRE) != 0, [] {
+    const bool early = (a.stages & STAGE_PRE) != 0;
+    if (early) order_acquire(a.order, a.order_tag);   // each thread for its own reads
+    squirmer_update<S>(L, a, early, [] {
         pdl_wait();
         pdl_launch_dependents();
         return true;

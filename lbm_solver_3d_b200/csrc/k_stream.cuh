@@ -771,7 +771,7 @@ __host__ __device__ constexpr int bulk_min_blocks(bool dense) {
 template <class S, int PAR, bool SQ, bool MACRO, bool WR, bool DENSE = false>
 __global__ void __launch_bounds__(256, bulk_min_blocks<S>(DENSE)) k_bulk(const Lattice L, const StreamArgs a) {
     pdl_wait();
-    if (WR && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) order_publish(a.order, a.order_tag);
+    if (WR && (blockIdx.x | blockIdx.y | threadIdx.x) == 0) order_publish(a.order + ORDER_WALL, a.order_tag);
     pdl_launch_dependents();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     int y, z;
@@ -1216,6 +1216,7 @@ __device__ __forceinline__ void copy_sq_state(SqState* dst, const SqState* src) 
 template <class S, int PAR, bool SQ, bool MACRO>
 __global__ void __maxnreg__(ZONE_MAX_REGS) k_zone(const Lattice L, const StreamArgs a) {
     pdl_wait();
+    if (SQ && (blockIdx.x | threadIdx.x) == 0) order_publish(a.order + ORDER_ZONE, a.order_tag);
     pdl_launch_dependents();
     __shared__ __align__(16) SqState zsq;
     __shared__ ZoneWarp<S> zw[BOUNDARY_BLOCK / 32];

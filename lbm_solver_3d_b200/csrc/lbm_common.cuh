@@ -245,8 +245,8 @@ struct StreamArgs {
     int apply_corr;               // add the pending correction on load (after one)
     int* row_claim;               // staged-row bulk: row counter and CTAs done (RowsWork)
     int late_wait;                // the bulk follows this step's wall rows and runs beside them (bulk_begin)
-    int* order;                   // word that the wall rows publish for such a bulk (order_publish), and
-    int order_tag;                // this step's value of it: differs from the two steps' before and after
+    int* order;                   // words that the wall rows publish for such a bulk, the zone for the squirmer
+    int order_tag;                // update (order_publish); this step's value differs from those of the steps around it
 };
 
 // ---- ensembles (k_batch.cuh) -------------------------------------------------
@@ -267,6 +267,7 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // step's tag (release), and a thread of the later kernel that reads that tag
 // (acquire) sees all that was visible there. One that does not find it waits
 // itself, so neither ever spins.
+constexpr int ORDER_WALL = 0, ORDER_ZONE = 1, ORDER_WORDS = 2;
 __device__ __forceinline__ void order_publish(int* word, int tag) {
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(word), "r"(tag) : "memory");
 }
@@ -285,7 +286,7 @@ __device__ __forceinline__ void order_acquire(const int* word, int tag) {
 // the CTA calls both.
 __device__ __forceinline__ void bulk_begin(const StreamArgs& a, bool late) {
     if (late) {
-        if (threadIdx.x == 0) order_acquire(a.order, a.order_tag);
+        if (threadIdx.x == 0) order_acquire(a.order + ORDER_WALL, a.order_tag);
         __syncthreads();
     } else {
         pdl_wait();

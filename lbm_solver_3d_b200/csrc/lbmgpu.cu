@@ -228,7 +228,7 @@ bool is_corr_step(const lbmgpu_handle* h, long long s) {
 // Words behind row_claim that one kernel of a step publishes for the next, and
 // the step's value: a function of what a captured step keeps, different from
 // that of the steps around it. Zero after a load, whose steps may repeat one.
-constexpr int ORDER_WALL = 2, ROW_WORDS = 3;
+constexpr int ROW_ORDER = 2, ROW_WORDS = ROW_ORDER + ORDER_WORDS;
 int order_tag(const StepPlan& sp) { return 1 + 2 * sp.zslot + sp.par; }
 
 StreamArgs stream_args(lbmgpu_handle* h, const StepPlan& sp) {
@@ -243,7 +243,7 @@ StreamArgs stream_args(lbmgpu_handle* h, const StepPlan& sp) {
     a.zslot = sp.zslot; a.do_mass = sp.corr ? 1 : 0; a.apply_corr = sp.apply ? 1 : 0;
     a.row_claim = h->row_claim;
     a.late_wait = 0;
-    a.order = h->row_claim + ORDER_WALL;
+    a.order = h->row_claim + ROW_ORDER;
     a.order_tag = order_tag(sp);
     return a;
 }
@@ -259,6 +259,8 @@ SqArgs squirmer_args(lbmgpu_handle* h, int parity, int stages, int corr_step, in
     a.chg_cap = h->chg_cap; a.shell = h->shell; a.shell_hdr = h->shell_hdr;
     a.traj = h->traj; a.sq = h->sq; a.parity = parity; a.stages = stages;
     a.corr_step = corr_step; a.zslot_a = za; a.zslot_b = zb;
+    a.order = h->row_claim + ROW_ORDER + ORDER_ZONE;
+    a.order_tag = 0;
     return a;
 }
 
@@ -566,8 +568,10 @@ void issue_fused(lbmgpu_handle* h, cudaStream_t sa, cudaStream_t sb, const StepP
     if (h->has_sq) {
         if (sp.corr) cudaStreamWaitEvent(sb, h->ev_b[sp.s & 1], 0);
         const int za = (int)((sp.s + 2) % ZONE_SLOTS);
-        h->lz->squirmer(h->L, squirmer_args(h, par ^ 1, STAGE_PRE | STAGE_FORCE | STAGE_BODY | STAGE_REMAP | STAGE_LOOP,
-                                            sp.corr ? 1 : 0, za, -1), sb);
+        SqArgs q = squirmer_args(h, par ^ 1, STAGE_PRE | STAGE_FORCE | STAGE_BODY | STAGE_REMAP | STAGE_LOOP,
+                                 sp.corr ? 1 : 0, za, -1);
+        q.order_tag = a.order_tag;
+        h->lz->squirmer(h->L, q, sb);
         cudaEventRecord(h->ev_s, sb);
         ++k;
     }
@@ -1432,7 +1436,7 @@ int lbmgpu_checkpoint_load(lbmgpu_handle* h, const void* buf, size_t len) {
         // which candidates are tested)
         CUDA_TRY(h, cudaMemsetAsync(h->shell_hdr, 0, sizeof(ShellCache), st));
     }
-    CUDA_TRY(h, cudaMemsetAsync(h->row_claim + ORDER_WALL, 0, (ROW_WORDS - ORDER_WALL) * sizeof(int), st));
+    CUDA_TRY(h, cudaMemsetAsync(h->row_claim + ROW_ORDER, 0, ORDER_WORDS * sizeof(int), st));
     CUDA_TRY(h, cudaStreamSynchronize(st));
     CUDA_TRY(h, cudaGetLastError());
     h->t_main = hd.t_main;
