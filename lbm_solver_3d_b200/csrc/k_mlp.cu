@@ -43,8 +43,14 @@
 #include <vector>
 
 #include "../../include/lbmgpu.h"
+#include "pdl.cuh"
 
 namespace {
+
+using lbmgpu::order_acquire;
+using lbmgpu::order_publish;
+using lbmgpu::pdl_launch_dependents;
+using lbmgpu::pdl_wait;
 
 constexpr int NI = LBMGPU_MLP_IN, NH = LBMGPU_MLP_HIDDEN, NO = LBMGPU_MLP_OUT;
 constexpr int NP = LBMGPU_MLP_NPARAMS;
@@ -157,9 +163,6 @@ __device__ __forceinline__ void put2(__nv_bfloat16* p, float a, float b) { *rein
 __device__ __forceinline__ void put1(float* p, float a) { *p = a; }
 __device__ __forceinline__ void put1(__nv_bfloat16* p, float a) { *p = __float2bfloat16_rn(a); }
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // A 64-wide weight matrix of `rows` rows (rows >= valid are zero) into its padded place.
 template <int SH, class T>
 __device__ __forceinline__ void load_w64(T* dst, const float* w, int rows, int valid) {
@@ -175,14 +178,14 @@ __device__ __forceinline__ void load_w64(T* dst, const float* w, int rows, int v
 //   X [n][4], Yt [n][3] (targets, TRAIN), idx: sample order (NULL: identity);
 //   TRAIN: one tile per CTA of 2 MLP_THREADS; grad_part[blockIdx.x][NPS] and
 //          loss_part[blockIdx.x] = sum of squared errors of the tile;
-//          dL/dY = 2 (Y - Yt) * inv_count;
+//          dL/dY = 2 (Y - Yt) * inv_count; order, tag: published for k_mlp_adam;
 //   else:  Yout [n][3]; a CTA of MLP_THREADS takes tiles blockIdx.x, + gridDim.x,
 //          ... with the parameters loaded once.
 template <bool BF16, bool TRAIN>
 __global__ void __launch_bounds__(TRAIN ? 2 * MLP_THREADS : MLP_THREADS)
     k_mlp_tile(const float* params, const float* __restrict__ X, const float* __restrict__ Yt,
                const int* __restrict__ idx, int base, int n, float inv_count, float* __restrict__ grad_part,
-               float* __restrict__ loss_part, float* __restrict__ Yout) {
+               float* __restrict__ loss_part, float* __restrict__ Yout, int* order, int tag) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using Sm = Smem<BF16>;
     constexpr int SH = Sm::SH, SI = Sm::SI;
@@ -197,22 +200,25 @@ __global__ void __launch_bounds__(TRAIN ? 2 * MLP_THREADS : MLP_THREADS)
     for (int tile = blockIdx.x;; tile += gridDim.x) {
     const int t0 = base + tile * MLP_T;   // first sample slot of this tile
     if (!TRAIN && t0 >= n) break;
-    // inputs (static while the optimizer runs: before the wait), padded
+    // inputs, padded; before the wait: they were copied before the first of the
+    // call's kernels was launched and are static since (read past the L1, which
+    // may hold an earlier call's)
     float yt = 0.f, yt2 = 0.f;            // TRAIN: this thread's targets
     if (tid < MLP_T * PI_) {
         const int s = tid / PI_, k = tid % PI_, slot = t0 + s;
         float v = 0.f;
-        if (k < NI && slot < n) v = X[(size_t)(idx ? idx[slot] : slot) * NI + k];
+        if (k < NI && slot < n) v = __ldcg(X + (size_t)(idx ? __ldcg(idx + slot) : slot) * NI + k);
         put1(S.H0 + s * SI + k, v);
         if (TRAIN && tid < LOSS_THREADS) {
             const int s2 = (tid + LOSS_THREADS) / PO, o = tid % PO;
-            if (o < NO && t0 + s < n) yt = Yt[(size_t)(idx ? idx[t0 + s] : t0 + s) * NO + o];
-            if (o < NO && t0 + s2 < n) yt2 = Yt[(size_t)(idx ? idx[t0 + s2] : t0 + s2) * NO + o];
+            if (o < NO && t0 + s < n) yt = __ldcg(Yt + (size_t)(idx ? __ldcg(idx + t0 + s) : t0 + s) * NO + o);
+            if (o < NO && t0 + s2 < n) yt2 = __ldcg(Yt + (size_t)(idx ? __ldcg(idx + t0 + s2) : t0 + s2) * NO + o);
         }
     }
     if (TRAIN || tile == (int)blockIdx.x) {
         if (TRAIN) {
             pdl_wait();
+            if (blockIdx.x == 0 && tid == 0) order_publish(order, tag);
             pdl_launch_dependents();
         }
         // parameters, padded
@@ -371,17 +377,21 @@ __global__ void __launch_bounds__(TRAIN ? 2 * MLP_THREADS : MLP_THREADS)
 
 // Sum of the tile partials (tile order) and one Adam step. With lr = 0 only
 // the gradient (and loss) is produced. The optimizer's state was last written
-// by the Adam step before the tiles, which waited for it: it is fetched before
-// this kernel's own wait. The last CTA sums the loss.
+// by the Adam step before the tiles, which waited for it and published tag: it
+// is fetched before this kernel's own wait. The last CTA sums the loss.
 constexpr int ADAM_THREADS = 128, ADAM_GRID = (NP + ADAM_THREADS - 1) / ADAM_THREADS;
 __global__ void __launch_bounds__(ADAM_THREADS) k_mlp_adam(float* __restrict__ params, float* __restrict__ m1,
                                                            float* __restrict__ m2, const float* grad_part, int nparts,
                                                            const float* loss_part, float inv_count, float lr,
                                                            float beta1, float beta2, float eps, float bc1, float bc2,
-                                                           float* __restrict__ grad_out, float* __restrict__ loss_out) {
+                                                           float* __restrict__ grad_out, float* __restrict__ loss_out,
+                                                           const int* order, int tag) {
     const int p = blockIdx.x * ADAM_THREADS + threadIdx.x;
     float w = 0.f, a = 0.f, b = 0.f;
-    if (p < NP && lr != 0.f) { w = __ldcg(params + p); a = __ldcg(m1 + p); b = __ldcg(m2 + p); }
+    if (p < NP && lr != 0.f) {
+        order_acquire(order, tag);
+        w = __ldcg(params + p); a = __ldcg(m1 + p); b = __ldcg(m2 + p);
+    }
     pdl_wait();
     pdl_launch_dependents();
     if (blockIdx.x == ADAM_GRID) {
@@ -652,7 +662,8 @@ struct lbmgpu_mlp {
     float *xin = nullptr, *yout = nullptr;
     int xin_cap = 0, yout_cap = 0;      // floats
     float* small = nullptr;             // [0] loss, [1..NP] gradient
-    int* d_err = nullptr;               // tensor-core forward: a bounded wait gave up
+    int* d_err = nullptr;               // tensor-core forward: a bounded wait gave up; then the order word (pdl.cuh)
+    unsigned batches = 0;               // minibatches launched: the order word's value
     long long t = 0;                    // Adam steps taken
     float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
     std::string err;
@@ -718,10 +729,11 @@ int train_batch(lbmgpu_mlp* m, const int* idx, int base, int count, float lr, fl
     int rc = ensure_parts(m, tiles);
     if (rc) return rc;
     const float inv = 1.0f / (float)(count * NO);
+    const int tag = (int)++m->batches;   // another value than the minibatch before left
     // the tile kernel sees slots [base, base + count) of idx as its samples
     MTRY(m, launch_pdl(m->bf16 ? k_mlp_tile<true, true> : k_mlp_tile<false, true>, tiles, 2 * MLP_THREADS,
                        m->bf16 ? sizeof(Smem<true>) : sizeof(Smem<false>), m->stream, (const float*)m->params, (const float*)m->X, (const float*)m->Y, idx, base,
-                       base + count, inv, m->grad_part, m->loss_part, (float*)nullptr));
+                       base + count, inv, m->grad_part, m->loss_part, (float*)nullptr, m->d_err + 1, tag));
     float bc1 = 1.f, bc2 = 1.f;
     if (lr > 0.f) {
         m->t += 1;
@@ -730,7 +742,7 @@ int train_batch(lbmgpu_mlp* m, const int* idx, int base, int count, float lr, fl
     }
     MTRY(m, launch_pdl(k_mlp_adam, ADAM_GRID + 1, ADAM_THREADS, 0, m->stream, m->params, m->m1, m->m2,
                        (const float*)m->grad_part, tiles, (const float*)m->loss_part, inv, lr, m->beta1, m->beta2,
-                       m->eps, bc1, bc2, d_grad, d_loss));
+                       m->eps, bc1, bc2, d_grad, d_loss, (const int*)(m->d_err + 1), tag));
     return LBMGPU_OK;
 }
 
@@ -762,8 +774,8 @@ int lbmgpu_mlp_create(int device, int bf16, lbmgpu_mlp** out) {
     if ((e = cudaMalloc(&m->m1, NP * sizeof(float))) != cudaSuccess) return bail(e, "cudaMalloc");
     if ((e = cudaMalloc(&m->m2, NP * sizeof(float))) != cudaSuccess) return bail(e, "cudaMalloc");
     if ((e = cudaMalloc(&m->small, (NP + 1) * sizeof(float))) != cudaSuccess) return bail(e, "cudaMalloc");
-    if ((e = cudaMalloc(&m->d_err, sizeof(int))) != cudaSuccess) return bail(e, "cudaMalloc");
-    if ((e = cudaMemsetAsync(m->d_err, 0, sizeof(int), m->stream)) != cudaSuccess) return bail(e, "memset");
+    if ((e = cudaMalloc(&m->d_err, 2 * sizeof(int))) != cudaSuccess) return bail(e, "cudaMalloc");
+    if ((e = cudaMemsetAsync(m->d_err, 0, 2 * sizeof(int), m->stream)) != cudaSuccess) return bail(e, "memset");
     if ((e = cudaMemsetAsync(m->params, 0, NP * sizeof(float), m->stream)) != cudaSuccess) return bail(e, "memset");
     if ((e = cudaMemsetAsync(m->m1, 0, NP * sizeof(float), m->stream)) != cudaSuccess) return bail(e, "memset");
     if ((e = cudaMemsetAsync(m->m2, 0, NP * sizeof(float), m->stream)) != cudaSuccess) return bail(e, "memset");
@@ -898,10 +910,10 @@ int lbmgpu_mlp_forward_ex(lbmgpu_mlp* m, const float* x, int n, float* y, int pa
         const size_t sm = m->bf16 ? sizeof(Smem<true>) : sizeof(Smem<false>);
         if (m->bf16)
             k_mlp_tile<true, false><<<tiles, MLP_THREADS, sm, m->stream>>>(m->params, m->xin, nullptr, nullptr, 0, n,
-                                                                           0.f, nullptr, nullptr, m->yout);
+                                                                           0.f, nullptr, nullptr, m->yout, nullptr, 0);
         else
             k_mlp_tile<false, false><<<tiles, MLP_THREADS, sm, m->stream>>>(m->params, m->xin, nullptr, nullptr, 0, n,
-                                                                            0.f, nullptr, nullptr, m->yout);
+                                                                            0.f, nullptr, nullptr, m->yout, nullptr, 0);
     }
     MTRY(m, cudaGetLastError());
     int err = 0;

@@ -7,6 +7,8 @@
 #include <cstdint>
 #include <cuda_fp16.h>
 
+#include "pdl.cuh"
+
 namespace lbmgpu {
 
 // ---- D3Q19, in the reference's order (src/utils/lattice.hpp:18-30) --------
@@ -252,30 +254,7 @@ struct StreamArgs {
 // ---- ensembles (k_batch.cuh) -------------------------------------------------
 constexpr int BATCH_MAX_NX = 256;   // longest x-row of an ensemble member
 
-// Programmatic dependent launch. A kernel launched with programmatic stream
-// serialisation may start before its predecessor in the stream has finished;
-// pdl_wait() blocks until that predecessor has completed and its writes are
-// visible, so it comes before the first read of anything the predecessor
-// writes. pdl_launch_dependents() lets the successor start early. Both are
-// no-ops for an ordinary launch.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// What a kernel that waits for its predecessor is shown, a kernel behind it that
-// has not waited yet is not: pdl_wait makes earlier writes visible to the grid
-// that calls it. A thread behind its own pdl_wait therefore publishes this
-// step's tag (release), and a thread of the later kernel that reads that tag
-// (acquire) sees all that was visible there. One that does not find it waits
-// itself, so neither ever spins.
-constexpr int ORDER_WALL = 0, ORDER_ZONE = 1, ORDER_WORDS = 2;
-__device__ __forceinline__ void order_publish(int* word, int tag) {
-    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(word), "r"(tag) : "memory");
-}
-__device__ __forceinline__ void order_acquire(const int* word, int tag) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
-    if (v != tag) pdl_wait();
-}
+constexpr int ORDER_WALL = 0, ORDER_ZONE = 1, ORDER_WORDS = 2;   // words of StreamArgs::order
 
 // Start and end of a bulk kernel. Usually it waits for its predecessor, the
 // bulk of the step before. Where the wall rows of the same step are launched
