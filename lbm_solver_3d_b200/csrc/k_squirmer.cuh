@@ -894,7 +894,7 @@ __device__ __forceinline__ BodyPre body_pre(const Lattice& L, const SqState& s, 
     b.c = warp == 0 ? s.Fc[d] : s.Tc[d];
     b.M = warp == 0 ? s.M : s.I;
     b.y = 1.0 / b.M;
-    b.yfar = exponent_far(b.M) || b.M == 0.0;
+    b.yfar = divisor_far(b.M);
     b.e1 = s.e[d1]; b.e2 = s.e[d2];
     b.lo = 0.5 + s.R + s.hmin; b.hi = (nd - 1.5) - s.R - s.hmin;
     b.base = d == 0 ? shell_X[0] : (d == 1 ? shell_X[1] : shell_X[2]);
@@ -906,7 +906,7 @@ __device__ __forceinline__ void body_rotation(SqShared& sh, const BodyPre& b, do
     constexpr unsigned ALL = 0xffffffffu;
     const int d1 = d == 2 ? 0 : d + 1, d2 = d == 0 ? 2 : d - 1;
     // Squirmer::integrate (squirmer.cpp:52-68)
-    double w = b.v + div_by(T + b.c, b.M, b.y, exponent_far(T + b.c) || b.yfar), e = b.X;
+    double w = b.v + div_by(T + b.c, b.M, b.y, numerator_far(T + b.c) || b.yfar), e = b.X;
     if (b.planar && d != 2) w = 0.0;
     e += __shfl_sync(ALL, w, d1) * b.e2 - __shfl_sync(ALL, w, d2) * b.e1;
     if (b.planar && d == 2) e = 0.0;
@@ -933,7 +933,7 @@ __device__ __forceinline__ void body_motion(const Lattice& L, SqShared& sh, cons
             if (hu < b.hc) Fw -= soft_wall_force(hu, s.eps, s.FS, b.hc);
         }
         // Squirmer::integrate (squirmer.cpp:52-68)
-        double v = b.v + div_by(F + b.c + Fw, b.M, b.y, exponent_far(F + b.c + Fw) || b.yfar);
+        double v = b.v + div_by(F + b.c + Fw, b.M, b.y, numerator_far(F + b.c + Fw) || b.yfar);
         if (b.planar && d == 2) v = 0.0;
         X += v;
         int hits = 0;

@@ -244,22 +244,27 @@ struct HeldSrc {
 // a / b, correctly rounded, given y = 1 / b correctly rounded (Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor",
 // 1990): the residual of a y is exact in one FMA and the corrected quotient
-// rounds as the division does. far: a or b may be outside the range where that
-// holds (see exponent_far), and the division itself decides.
+// rounds as the division does, zeros with their sign. far: a or b is outside
+// the range where that holds and nothing on the way under- or overflows
+// (numerator_far, divisor_far), and the division itself decides.
 __device__ __forceinline__ double div_by(double a, double b, double y, bool far) {
     if (far) return a / b;
     const double q = __dmul_rn(a, y);
-    return __fma_rn(__fma_rn(-b, q, a), y, q);
+    return __fma_rn(-__fma_rn(q, b, -a), y, q);
 }
-// not zero and outside 2^-512 .. 2^512 (infinities and NaN included)
-__device__ __forceinline__ bool exponent_far(double a) {
+// not zero and outside 2^-500 .. 2^500 (infinities and NaN included)
+__device__ __forceinline__ bool numerator_far(double a) {
     const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
-    return hi - 0x1ff00000u >= 0x40000000u && (hi | (unsigned)__double2loint(a)) != 0u;
+    return hi - 0x20b00000u >= 0x3e800000u && (hi | (unsigned)__double2loint(a)) != 0u;
+}
+// not a positive number within 2^-500 .. 2^500
+__device__ __forceinline__ bool divisor_far(double b) {
+    return (unsigned)__double2hiint(b) - 0x20b00000u >= 0x3e800000u;
 }
 // (a0, a1, a2) / r: one division, the bits of three
 __device__ __forceinline__ void div3(double a0, double a1, double a2, double r, double& u, double& v, double& w) {
     const double y = 1.0 / r;
-    const bool far = exponent_far(r) || r == 0.0 || exponent_far(a0) || exponent_far(a1) || exponent_far(a2);
+    const bool far = divisor_far(r) || numerator_far(a0) || numerator_far(a1) || numerator_far(a2);
     u = div_by(a0, r, y, far);
     v = div_by(a1, r, y, far);
     w = div_by(a2, r, y, far);
