@@ -846,8 +846,8 @@ __global__ void __launch_bounds__(RUNS_THREADS, 2) k_bulk_runs(const Lattice* __
 //  ROWS_MAX_NX), persistent over the interior rows (y = ylo + r % nry,
 //  z = zlo + r / nry), which the producers claim one at a time from a counter
 //  (RowsWork): a CTA that starts late, or shares its SM with other kernels,
-//  takes fewer rows instead of ending late. CTAs that land on one of the
-//  `reserve` lowest-numbered SMs leave at once (rows_idle).
+//  takes fewer rows instead of ending late. The first CTAs that land on one of
+//  the `reserve` lowest-numbered SMs leave at once (rows_leave).
 //    producer   per row: claims the row, waits for the stage to be free
 //               (empty barrier), publishes the row number, then
 //               lane i < 19 copies direction-row i of the state -- A[i] of row
@@ -876,12 +876,15 @@ __host__ __device__ constexpr size_t rows_stage_bytes(int nx) {
 }
 
 // The interior rows of one launch and how CTAs share them. claim[0] is the
-// next unclaimed row, claim[1] the CTAs that have finished; the last CTA to
-// finish sets both back to 0 for the next launch, which stream order keeps
-// after this one.
+// next unclaimed row, claim[ROWS_DONE] the CTAs that have finished and
+// claim[ROWS_LEFT] those that asked to leave (rows_leave); the last CTA to
+// finish sets all back to 0 for the next launch, which stream order keeps
+// after this one. Each word has a line of its own: the claims of a launch's
+// start queue at theirs for some 2 us.
+constexpr int ROWS_DONE = 64, ROWS_LEFT = 128, ROWS_WORDS = 192;
 struct RowsWork {
     int nry, nrows, ylo, zlo;   // rows nry x (nrows / nry) from (ylo, zlo)
-    int reserve;                // CTAs on SMs with %smid < reserve take no rows
+    int reserve, idle;          // the first `idle` CTAs on SMs with %smid < reserve take no rows
     int* claim;
 };
 
@@ -893,11 +896,17 @@ __device__ __forceinline__ unsigned sm_id() {
 
 // A CTA on one of the reserved SMs takes no rows, so that the squirmer update
 // (one CTA of 512 threads, which needs an SM to itself) finds one free while
-// the persistent grid runs -- except the grid's last CTA, so that the rows are
-// done whatever the placement (the claim counter lets one CTA finish them
-// all). Uniform over the CTA.
-__device__ __forceinline__ bool rows_idle(const RowsWork& w) {
-    return (int)sm_id() < w.reserve && blockIdx.x + 1 < gridDim.x;
+// the persistent grid runs -- except the grid's last CTA. The CTAs that find no
+// place at first (other kernels hold part of the chip) follow those that left
+// onto the reserved SMs, so only `idle` of the grid may leave, an eighth of it:
+// without a bound, where a second lattice was stepped beside this one, nearly
+// all did. Two 192x96x96 FP32 slits from two threads took 300 to 1,300 us a
+// step, 129 with the bound; two 256x128x128 FP16 560 to 1,400, 165. A bound of
+// what the reserved SMs hold at a time kept them busy behind wall rows in front
+// of the bulk: 128x64x64 FP32 26.7 us a step, 24.2 with an eighth, as without
+// a bound. For one thread of the CTA.
+__device__ __forceinline__ bool rows_leave(const RowsWork& w) {
+    return (int)sm_id() < w.reserve && atomicAdd(w.claim + ROWS_LEFT, 1) < w.idle;
 }
 
 // Populations of node x from a staged row (whole direction-rows of nx elements;
@@ -1010,9 +1019,10 @@ __device__ __forceinline__ void rows_finish(const RowsWork& w, uint64_t* full, v
                 mbar_wait(&full[q], (uint32_t)(((issued - q + NST - 1) / NST - 1) & 1));
         }
         __threadfence();
-        if (atomicAdd(w.claim + 1, 1) == (int)gridDim.x - 1) {
+        if (atomicAdd(w.claim + ROWS_DONE, 1) == (int)gridDim.x - 1) {
             w.claim[0] = 0;
-            w.claim[1] = 0;
+            w.claim[ROWS_DONE] = 0;
+            w.claim[ROWS_LEFT] = 0;
             __threadfence();
         }
     }
@@ -1033,6 +1043,7 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX, RowsCfg<S>::MINB) k_bulk_row
     __shared__ int rowid[NST];                                     // the row in stage q (-1: none left)
     __shared__ volatile int s_abort;
     __shared__ int s_issued;
+    __shared__ bool s_idle;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nx = L.nx, nupd = nx >> 5;
     const size_t stage = rows_stage_bytes<S>(nx);
@@ -1047,10 +1058,11 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX, RowsCfg<S>::MINB) k_bulk_row
         s_abort = 0;
         s_issued = 0;
         if (SQ) zb = a.sq->zone[a.zslot];
+        s_idle = rows_leave(w);
     }
     __syncthreads();
 
-    if (rows_idle(w)) {
+    if (s_idle && blockIdx.x + 1 < gridDim.x) {
     } else if (warp == 0) {
         rows_produce<S, PAR, NST>(L, a, w, rows_raw, stage, full, empty, rowid, s_abort, s_issued, lane);
     } else {
@@ -1146,6 +1158,7 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX / 2, Rows2Cfg<S>::MINB) k_bul
     __shared__ int rowid[NST];
     __shared__ volatile int s_abort;
     __shared__ int s_issued;
+    __shared__ bool s_idle;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nx = L.nx, nupd = nx >> 6;
     const size_t stage = rows_stage_bytes<S>(nx);
@@ -1159,10 +1172,11 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX / 2, Rows2Cfg<S>::MINB) k_bul
         s_abort = 0;
         s_issued = 0;
         if (SQ) zb = a.sq->zone[a.zslot];
+        s_idle = rows_leave(w);
     }
     __syncthreads();
 
-    if (rows_idle(w)) {
+    if (s_idle && blockIdx.x + 1 < gridDim.x) {
     } else if (warp == 0) {
         rows_produce<S, PAR, NST>(L, a, w, rows_raw, stage, full, empty, rowid, s_abort, s_issued, lane);
     } else {

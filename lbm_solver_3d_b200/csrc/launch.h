@@ -27,6 +27,7 @@ struct StreamGeom {
     int rows_nry = 0, rows_n = 0, rows_ylo = 0, rows_zlo = 0;
     bool rows_pairs = false;   // two nodes per update thread (k_bulk_rows2)
     int rows_reserve = 0;      // SMs (lowest %smid) the rows grid leaves to the zone and squirmer kernels
+    int rows_idle = 0;         // CTAs that may leave for it (rows_leave)
 };
 
 struct SqArgs;

@@ -245,7 +245,7 @@ struct StreamArgs {
     int zslot;                    // zone slot of this step
     int do_mass;                  // sum the stored populations (a correction step)
     int apply_corr;               // add the pending correction on load (after one)
-    int* row_claim;               // staged-row bulk: row counter and CTAs done (RowsWork)
+    int* row_claim;               // staged-row bulk: its counters (RowsWork)
     int late_wait;                // the bulk follows this step's wall rows and runs beside them (bulk_begin)
     int* order;                   // words that the wall rows publish for such a bulk, the zone for the squirmer
     int order_tag;                // update (order_publish); this step's value differs from those of the steps around it

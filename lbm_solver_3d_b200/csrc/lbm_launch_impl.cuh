@@ -49,7 +49,7 @@ static void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
 template <class S, int PAR, bool SQ, bool MACRO>
 static void bulk_one(const Lattice& L, const StreamArgs& a, const StreamGeom& g, cudaStream_t st) {
     if (g.rows_grid) {   // rows staged in shared memory (every step; sums in k_bulk's order)
-        const RowsWork w{g.rows_nry, g.rows_n, g.rows_ylo, g.rows_zlo, g.rows_reserve, a.row_claim};
+        const RowsWork w{g.rows_nry, g.rows_n, g.rows_ylo, g.rows_zlo, g.rows_reserve, g.rows_idle, a.row_claim};
         if constexpr (S::shifted && !MACRO) {
             if (g.rows_pairs && !a.do_mass) {   // no sums this step: two nodes per update thread
                 launch_pdl(k_bulk_rows2<S, PAR, SQ>, dim3(g.rows_grid), dim3(32 + L.nx / 2), rows2_smem<S>(L.nx), st, L, a, w);

@@ -83,7 +83,7 @@ struct lbmgpu_handle {
     unsigned nblocks = 0;
     double* block_part_b = nullptr;
     unsigned nblocks_b = 0;
-    int* row_claim = nullptr;      // staged-row bulk: row counter, CTAs done; then the order words (order_publish)
+    int* row_claim = nullptr;      // staged-row bulk's counters (RowsWork), then the order words (order_publish)
     int* ordermap = nullptr;
     int* chg_node = nullptr;
     int* chg_key = nullptr;
@@ -225,10 +225,10 @@ bool is_corr_step(const lbmgpu_handle* h, long long s) {
     return h->has_sq && k > 0 && s % k == 0;
 }
 
-// Words behind row_claim that one kernel of a step publishes for the next, and
+// Words behind row_claim's that one kernel of a step publishes for the next, and
 // the step's value: a function of what a captured step keeps, different from
 // that of the steps around it. Zero after a load, whose steps may repeat one.
-constexpr int ROW_ORDER = 2, ROW_WORDS = ROW_ORDER + ORDER_WORDS;
+constexpr int ROW_ORDER = ROWS_WORDS, ROW_WORDS = ROW_ORDER + ORDER_WORDS;
 int order_tag(const StepPlan& sp) { return 1 + 2 * sp.zslot + sp.par; }
 
 StreamArgs stream_args(lbmgpu_handle* h, const StepPlan& sp) {
@@ -834,6 +834,7 @@ int create_impl(const lbmgpu_params* p, const MemberOpts* mo, lbmgpu_handle** ou
                 h->geom.rows_reserve = rows_reserve(h->has_sq != 0, h->geom.nwallrows > 0, sms, pairs,
                                                     per_sm * (1 + p->nx / (pairs ? 64 : 32)),
                                                     (double)Q * 2.0 * h->esize * (double)N);
+                h->geom.rows_idle = std::max(h->geom.rows_reserve * per_sm, (int)h->geom.rows_grid / 8);
             }
         }
     }
