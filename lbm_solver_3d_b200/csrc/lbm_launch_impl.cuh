@@ -70,9 +70,19 @@ static void bulk_one(const Lattice& L, const StreamArgs& a, const StreamGeom& g,
         }
     }
     if (!MACRO && !a.do_mass && g.flat.x) {   // no sums this step: whole rows of nodes per block
-        if (a.late_wait) launch_pdl(k_bulk_flat<S, PAR, SQ, false, true>, g.flat, dim3(256), 0, st, L, a);
-        else if (!S::shifted && g.dense) k_bulk_flat<S, PAR, SQ, true><<<g.flat, 256, 0, st>>>(L, a);
-        else k_bulk_flat<S, PAR, SQ><<<g.flat, 256, 0, st>>>(L, a);
+        if constexpr (SQ) {   // wall rows go in front of the bulk only where a squirmer's chain is the step
+            if (a.late_wait) {
+                launch_pdl(k_bulk_flat<S, PAR, SQ, false, true>, g.flat, dim3(256), 0, st, L, a);
+                return;
+            }
+        }
+        if constexpr (!S::shifted) {
+            if (g.dense) {
+                k_bulk_flat<S, PAR, SQ, true><<<g.flat, 256, 0, st>>>(L, a);
+                return;
+            }
+        }
+        k_bulk_flat<S, PAR, SQ><<<g.flat, 256, 0, st>>>(L, a);
         return;
     }
     if constexpr (!S::shifted) {
