@@ -1047,7 +1047,8 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX, RowsCfg<S>::MINB) k_bulk_row
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nx = L.nx, nupd = nx >> 5;
     const size_t stage = rows_stage_bytes<S>(nx);
-    bulk_begin(a, a.late_wait != 0);
+    if (!a.late_wait) pdl_wait();
+    pdl_launch_dependents();
     if (tid == 0) {
         for (int q = 0; q < NST; ++q) {
             mbar_init(&full[q], 1);
@@ -1057,6 +1058,7 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX, RowsCfg<S>::MINB) k_bulk_row
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
         s_issued = 0;
+        if (a.late_wait) order_acquire(a.order + ORDER_WALL, a.order_tag);   // see bulk_begin
         if (SQ) zb = a.sq->zone[a.zslot];
         s_idle = rows_leave(w);
     }
@@ -1162,7 +1164,8 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX / 2, Rows2Cfg<S>::MINB) k_bul
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nx = L.nx, nupd = nx >> 6;
     const size_t stage = rows_stage_bytes<S>(nx);
-    bulk_begin(a, a.late_wait != 0);
+    if (!a.late_wait) pdl_wait();
+    pdl_launch_dependents();
     if (tid == 0) {
         for (int q = 0; q < NST; ++q) {
             mbar_init(&full[q], 1);
@@ -1171,6 +1174,7 @@ __global__ void __launch_bounds__(32 + ROWS_MAX_NX / 2, Rows2Cfg<S>::MINB) k_bul
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
         s_issued = 0;
+        if (a.late_wait) order_acquire(a.order + ORDER_WALL, a.order_tag);   // see bulk_begin
         if (SQ) zb = a.sq->zone[a.zslot];
         s_idle = rows_leave(w);
     }

@@ -262,7 +262,8 @@ constexpr int ORDER_WALL = 0, ORDER_ZONE = 1, ORDER_WORDS = 2;   // words of Str
 // let this kernel start, and the two touch disjoint slots: it starts at once,
 // with the wall rows' word for what came before them, and waits for them only
 // before it ends, so that its end still means the end of both. Every thread of
-// the CTA calls both.
+// the CTA calls both (the staged rows begin with the steps of bulk_begin
+// themselves, the thread that reads the word beside its other preparations).
 __device__ __forceinline__ void bulk_begin(const StreamArgs& a, bool late) {
     if (late) {
         if (threadIdx.x == 0) order_acquire(a.order + ORDER_WALL, a.order_tag);
