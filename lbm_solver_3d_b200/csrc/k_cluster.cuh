@@ -3,7 +3,7 @@
 //  launch, with the populations in the shared memory of one thread-block cluster.
 //
 //  A step of such a lattice by separate kernels is two launches and a chain of
-//  global round trips for a few thousand nodes: 4.0 us for the 4x34x34 FP64 duct,
+//  global round trips for a few thousand nodes: 3.4 us for the 4x34x34 FP64 duct,
 //  whose 0.7 MB of populations would cross HBM in 0.1 us. Here a cluster of up to
 //  16 CTAs holds them (each CTA the whole x-rows [rank * rows, + rows) of the
 //  lattice, wall layers included, A[i][node] as in global memory), a node's
@@ -16,8 +16,8 @@
 //  the fields and sums the wall force, runs by the separate kernels.
 //  Bound: instruction issue and the FP64 pipe of the few SMs, then the barrier
 //  and one remote latency a step. Against the separate kernels (us a step, FP64 /
-//  FP32 / FP16): 4x34x34 2.2 / 1.9 / 1.4 against 3.4 / 3.1 / 3.6; 8x32x32, the
-//  largest (512 nodes per CTA), 2.9 / 2.4 / 1.7 against 3.6 / 3.3 / 3.6; with two
+//  FP32 / FP16): 4x34x34 2.2 / 1.9 / 1.4 against 3.4 / 3.1 / 3.7; 8x32x32, the
+//  largest (512 nodes per CTA), 2.9 / 2.4 / 1.7 against 3.5 / 3.2 / 3.6; with two
 //  nodes per thread (16x32x32) it was 5.6 against 3.9, hence the limit of one.
 // ============================================================================
 #pragma once

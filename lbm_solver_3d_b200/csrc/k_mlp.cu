@@ -86,10 +86,11 @@ struct Smem {
     float red[LOSS_THREADS / 32];
 };
 
-// 1 / x for x >= 1, correctly rounded: the hardware's approximation and one
-// Newton step whose residual is exact in an FMA (Markstein 1990). Equal to the
-// division for every float in [1, 2^100) (compared over all of them); beyond
-// that, and for infinities and NaN, the division itself.
+// 1 / x for x >= 1, as the division rounds it: the hardware's approximation and
+// one Newton step whose residual is exact in an FMA (as Markstein 1990 corrects
+// quotients). The approximation's error has no bound from which equality would
+// follow; the test compares every float in [1, 2^100). Beyond that, and for
+// infinities and NaN, the division itself.
 __device__ __forceinline__ float recip_ge1(float x) {
     if (!(x < 1.2676506e30f)) return 1.0f / x;
     float y;
@@ -434,7 +435,8 @@ __global__ void __launch_bounds__(ADAM_THREADS) k_mlp_adam(float* __restrict__ p
 //  The grid is one wave of CTAs: each loads and rounds the weights once, holds
 //  its tensor memory, and takes tiles of 128 samples in turn. (With a CTA per
 //  tile the weights' 35 KB and their index arithmetic were most of the time:
-//  97 us for 250,001 samples, 76 us now; 42 -> 25 us for one tile.)
+//  98 us for 250,001 samples, 76 us now; 46 -> 24 us for one tile. A call is
+//  mostly its copies from and to pageable memory: 550 us for 250,001 samples.)
 //  Waits on the mbarrier are bounded; a timeout sets *err, and the tensor
 //  memory is released on every path.
 // ---------------------------------------------------------------------------

@@ -764,11 +764,12 @@ __host__ __device__ constexpr int bulk_min_blocks(bool dense) {
 //  squirmer update writes (except the correction value on the step after a
 //  correction step, when the launch waits for it).
 // ---------------------------------------------------------------------------
-//    DENSE (FP64 only) 3 CTAs/SM instead of 2 (80 registers, some spills): for
-//          long bulks; a short one leaves room for the zone and squirmer chain.
-//          The populations are loaded beside the type instead of after it
-//          (HeldSrc), although that spills 112 bytes: with 24 warps per SM the
-//          kernel is bound by those two latencies. Steps: 201x130x117 198.5 ->
+//    DENSE (FP64 only) 3 CTAs/SM instead of 2 (80 registers; odd steps spill 36
+//          to 52 bytes here and 16 in k_bulk_flat, even steps none): for long
+//          bulks; a short one leaves room for the zone and squirmer chain. The
+//          populations are loaded beside the type instead of after it
+//          (HeldSrc): with 24 warps per SM the kernel is bound by those two
+//          latencies. Steps: 201x130x117 198.5 ->
 //          178.4 us (0.72 -> 0.80 of the copy rate), 300x100x100 slit 194.1 ->
 //          177.2, 384x96x96 216.5 -> 202.5, 149x97x83 slit 87.9 -> 82.7. The
 //          shifted forms and the ensemble's chunks gained nothing from it (FP32

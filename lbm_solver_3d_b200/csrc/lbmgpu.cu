@@ -190,6 +190,9 @@ int bulk_kind() {
 //      FP64 201.9 -> 204.3.
 //   4  the FP16 two-node kernel (20 warps) from 170 MB: 256x128x128 96.4 ->
 //      92.0, 256x96x96 60.7 -> 57.0; 192x96x96 (134 MB) 50.2 -> 51.3.
+// The lines lie between the lattices named here, and all were stepped alone.
+// Where another lattice's kernels hold part of the chip, what counts is how many
+// CTAs may leave for it (rows_leave).
 int rows_reserve(bool squirmer, bool walls, int sms, bool pairs, int warps_per_sm, double bytes) {
     const char* e = std::getenv("LBMGPU_ROWS_RESERVE");
     int r = 2;
@@ -200,8 +203,8 @@ int rows_reserve(bool squirmer, bool walls, int sms, bool pairs, int warps_per_s
     return std::max(0, std::min(r, sms / 2));
 }
 
-// Steps per k_cluster_steps launch, at most (a launch of the smallest duct then
-// takes about a fifth of a second).
+// Steps per k_cluster_steps launch, at most (a launch for the 4x34x34 FP64 duct
+// then takes 0.3 s).
 constexpr int CLUSTER_MAX_STEPS = 1 << 17;
 
 // Capacity of the boundary-link list of a lattice with these parameters (the
