@@ -148,9 +148,11 @@ static void set_pop_launch(const Lattice& L, void* f, int P, int i, const double
 template <class S>
 static void correct_mass_launch(const Lattice& L, void* f, const uint8_t* flag, int P, SqState* sq, double* part,
                                 double* dflag, cudaStream_t st) {
-    k_mass_partial<S><<<MASS_GRID, AUX_BLOCK, 0, st>>>(L, f, flag, P, part);
+    if (P) k_mass_partial<S, 1><<<MASS_GRID, AUX_BLOCK, 0, st>>>(L, f, flag, part);
+    else k_mass_partial<S, 0><<<MASS_GRID, AUX_BLOCK, 0, st>>>(L, f, flag, part);
     k_mass_final<S><<<1, AUX_BLOCK, 0, st>>>(part, sq, dflag);
-    k_mass_apply<S><<<1184, AUX_BLOCK, 0, st>>>(L, f, flag, P, sq, dflag);
+    if (P) k_mass_apply<S, 1><<<1184, AUX_BLOCK, 0, st>>>(L, f, flag, sq, dflag);
+    else k_mass_apply<S, 0><<<1184, AUX_BLOCK, 0, st>>>(L, f, flag, sq, dflag);
 }
 
 template <class S, int PAR, bool MACRO, bool WR>
