@@ -44,7 +44,7 @@ constexpr int SQ_SORT_CAP = 2048;   // changes ordered in shared memory (3 ints 
 constexpr int SQ_GROUP = 4;         // remap candidates tested per thread with their loads in flight together
 constexpr int SQ_PRE = 8;           // candidates per thread fetched ahead: 4096 of them, the shell up to R = 9
 constexpr int SQ_FEW = 32;          // changed nodes that remap_few orders: one warp
-constexpr int SQ_FEW_LINKS = 4096;  // boundary links that remap_few edits in shared memory (R up to about 12)
+constexpr int SQ_FEW_LINKS = 4096;  // boundary links that remap_few edits in shared memory (R up to about 15)
 constexpr int STAGE_BODY = 1, STAGE_REMAP = 2, STAGE_LOOP = 4, STAGE_FORCE = 8;
 // The launch follows a zone kernel that had itself waited for the update before
 // and published order_tag: this update may read what that one wrote (its state,
@@ -471,10 +471,23 @@ __device__ __forceinline__ void remap_few(const Lattice& L, const SqArgs& a, SqS
 
 // The remap by the candidate list in full: rebuilds the list where needed,
 // orders any number of changes, and rebuilds the link list by walks over the
-// sphere's box. Off the usual path (remap_few), so it is kept out of line.
+// sphere's box. Off the usual path (remap_few) except for spheres of R > 15, so
+// it is kept out of line; what its walks use of its arguments is held locally,
+// since through the references every store might have changed it. A step of a
+// fast sphere (U = 0.005): R = 20 333 -> 262 us, R = 40 1,923 -> 1,491, with the
+// candidates of long link lists tested here only. (All arguments held locally:
+// 254 and 1,468, but a stack frame that costs every update 0.5 us.)
 template <class S>
-__device__ __noinline__ void remap_walk(const Lattice& L, const SqArgs& a, SqShared& sh, unsigned char* smem_raw,
-                                        int shell_ok, bool corr_step) {
+__device__ __noinline__ void remap_walk(const Lattice& lattice, const SqArgs& args, SqShared& sh, int shell_ok,
+                                        bool corr_step) {
+    Lattice L;
+    L.nx = lattice.nx; L.ny = lattice.ny; L.nz = lattice.nz; L.N = lattice.N; L.nxy = lattice.nxy;
+    L.walls_y = lattice.walls_y; L.walls_z = lattice.walls_z;
+    const SqArgs& a = args;
+    int* const a_shell = args.shell;
+    int* const a_cand = args.cand;
+    const int a_chg_cap = args.chg_cap;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     ChgSh* ch = reinterpret_cast<ChgSh*>(smem_raw);
     typedef cub::BlockScan<int, SQ_THREADS> Scan;
     SqState& s = sh.s;
@@ -552,12 +565,12 @@ __device__ __noinline__ void remap_walk(const Lattice& L, const SqArgs& a, SqSha
             box_walk([&](int, int x, int y, int z) {
                 const double r2 = approx_r2(x, y, z);
                 if (r2 >= Sin2 && r2 < Sout2) {
-                    if (off < a.chg_cap) a.shell[off] = x + L.nx * (y + L.ny * z);
+                    if (off < a_chg_cap) a_shell[off] = x + L.nx * (y + L.ny * z);
                     ++off;
                 }
             });
             if (tid == 0) {
-                sh_ncand = min(sh_total, a.chg_cap);
+                sh_ncand = min(sh_total, a_chg_cap);
                 ShellCache hc;
                 for (int d = 0; d < 3; ++d) hc.X[d] = s.X[d];
                 hc.n = sh_ncand;
@@ -576,7 +589,7 @@ __device__ __noinline__ void remap_walk(const Lattice& L, const SqArgs& a, SqSha
 #pragma unroll
             for (int g = 0; g < SQ_GROUP; ++g) {
                 const int c = c0 + g * SQ_THREADS;
-                nn[g] = c < ncand ? (unsigned)a.shell[c] : 0u;
+                nn[g] = c < ncand ? (unsigned)a_shell[c] : 0u;
             }
 #pragma unroll
             for (int g = 0; g < SQ_GROUP; ++g)
@@ -611,7 +624,7 @@ __device__ __noinline__ void remap_walk(const Lattice& L, const SqArgs& a, SqSha
             for (int c = c0; c < c1; ++c) {
                 const uint8_t mk = a.mark[c];
                 if (!mk) continue;
-                a.chg_node[off] = a.shell[c];
+                a.chg_node[off] = a_shell[c];
                 a.chg_key[off] = mk;
                 ++off;
             }
@@ -806,15 +819,15 @@ __device__ __noinline__ void remap_walk(const Lattice& L, const SqArgs& a, SqSha
             region_walk([&](int x, int y, int z) {
                 const double r2 = approx_r2(x, y, z);
                 if (r2 >= Lin2 && r2 < Lout2) {
-                    if (off < a.chg_cap) a.cand[off] = x + L.nx * (y + L.ny * z);
+                    if (off < a_chg_cap) a_cand[off] = x + L.nx * (y + L.ny * z);
                     ++off;
                 }
             });
         }
         __syncthreads();
-        const int nc2 = min(sh_total, a.chg_cap);
+        const int nc2 = min(sh_total, a_chg_cap);
         for (int c = tid; c < nc2; c += SQ_THREADS) {
-            const unsigned n = (unsigned)a.cand[c];
+            const unsigned n = (unsigned)a_cand[c];
             uint8_t mk = 0;
             if ((a.flag[n] & TYPE_MASK) == T_FLUID) {
                 const int x = (int)(n % (unsigned)L.nx), y = (int)((n / (unsigned)L.nx) % (unsigned)L.ny),
@@ -838,7 +851,7 @@ __device__ __noinline__ void remap_walk(const Lattice& L, const SqArgs& a, SqSha
             __syncthreads();
             for (int c = c0; c < c1; ++c) {
                 if (!a.mark[c]) continue;
-                const int n = a.cand[c];
+                const int n = a_cand[c];
                 if (off < a.link_cap) {
                     a.links[off] = n;
                     a.linkslot[n] = off;
@@ -1074,7 +1087,9 @@ __device__ __forceinline__ bool squirmer_update(const Lattice& L, const SqArgs& 
     // a lattice hardly wider than the sphere, where the offset may be about
     // half a lattice. If few nodes change, remap_few does the rest.
     if (remap) {
-        bool walk = sh.rebuild != 0;   // uniform
+        // A link list too long for remap_few would send every step with a change
+        // to the walk, which tests the candidates itself: at once then.
+        bool walk = sh.rebuild != 0 || s.n_links > SQ_FEW_LINKS;   // uniform
         if (!walk) {
             const double R2 = s.R * s.R;
             const float R2f = (float)R2, span = 2.0f * (float)s.R + 10.0f, ox = sh.off[0], oy = sh.off[1], oz = sh.off[2];
@@ -1108,8 +1123,8 @@ __device__ __forceinline__ bool squirmer_update(const Lattice& L, const SqArgs& 
         if (tid >= SQ_THREADS - 3) box_and_zones(L, a, sh, SQ_THREADS - 1 - tid);
         __syncthreads();
         const int nfew = sh.few;
-        walk = walk || (nfew > 0 && (nfew > SQ_FEW || shell_ok != 2 || s.n_links < 0 || s.n_links > SQ_FEW_LINKS));
-        if (walk) remap_walk<S>(L, a, sh, smem_raw, shell_ok, corr_step);   // uniform
+        walk = walk || (nfew > 0 && (nfew > SQ_FEW || shell_ok != 2 || s.n_links < 0));
+        if (walk) remap_walk<S>(L, a, sh, shell_ok, corr_step);   // uniform
         else if (nfew > 0) remap_few<S>(L, a, sh, fw, nfew, corr_step);
         if (tid == 0) s.n_fluid += sh.dfluid;
     }
